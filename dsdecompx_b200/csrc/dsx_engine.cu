@@ -769,6 +769,7 @@ struct dsx_grid {
         S.out_flags = device_alloc<int>(fixed_owned, P);
         S.list_len = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * E);
         S.send_base = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * E);
+        S.list_flat = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * E);
         S.g = device_alloc<int>(fixed_owned, P + 1);
         S.gbase = device_alloc<int>(fixed_owned, P + 1);
         cuda_check(cudaMemset(S.g, 0, sizeof(int) * (P + 1)), "memset");

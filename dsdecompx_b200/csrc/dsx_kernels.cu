@@ -764,16 +764,27 @@ __global__ void __launch_bounds__(NT) k_halo_classify(Grid G, const int4* __rest
     }
 }
 
+// Where sender r's 26 lists start in the order that walks the ghosts sender
+// by sender and list by list (one warp; `first`: ghosts of the senders before).
+__device__ __forceinline__ void write_list_flat(const int* list_len, int* list_flat, int r,
+                                                int first) {
+    const int lane = threadIdx.x & 31;
+    const int len = lane < kMaxNeighbors ? list_len[r * kMaxNeighbors + lane] : 0;
+    const int incl = warp_inclusive_sum(len);
+    if (lane < kMaxNeighbors) list_flat[r * kMaxNeighbors + lane] = first + incl - len;
+}
+
 // S2b: send-list lengths, receiver ghost layout (blocks in the receiver's
 // neighbor order, dsDecompX src/halo.cpp:609-649) and the first ghost slot of
 // every send list.  One CTA, one thread per receiver.
 __global__ void __launch_bounds__(1024) k_halo_layout(Grid G, const int* pre, int stride,
-                                                       int* list_len, int* send_base, int* gq,
-                                                       int* gbase, int* boff, int* info,
-                                                       int* cbase) {
+                                                       int* list_len, int* send_base,
+                                                       int* list_flat, int* gq, int* gbase,
+                                                       int* boff, int* info, int* cbase) {
     pdl_begin();
     __shared__ int ws[33];
     __shared__ int s_rcv[kMaxRanks + 1];
+    __shared__ int s_snd[kMaxRanks];
     const int P = G.P;
     const int ntiles = G.tile_start[P];
     for (int idx = threadIdx.x; idx < P * kMaxNeighbors; idx += blockDim.x) {
@@ -793,20 +804,29 @@ __global__ void __launch_bounds__(1024) k_halo_layout(Grid G, const int* pre, in
             len = e >= 0 ? list_len[e] : 0;
         }
         const int sum = __reduce_add_sync(0xffffffffu, len);
-        if (lane == 0) s_rcv[r] = sum;
+        const int sent = lane < kMaxNeighbors ? list_len[r * kMaxNeighbors + lane] : 0;
+        const int out = __reduce_add_sync(0xffffffffu, sent);
+        if (lane == 0) {
+            s_rcv[r] = sum;
+            s_snd[r] = out;
+        }
     }
     __syncthreads();
     const int q = threadIdx.x;
     const int mine = q < P ? s_rcv[q] : 0;
-    int total;
+    const int sent_all = q < P ? s_snd[q] : 0;
+    int total, total_sent;
     const int excl = block_scan_excl<1024>(mine, total, ws);
+    const int sent_excl = block_scan_excl<1024>(sent_all, total_sent, ws);
     if (q < P) {
         gq[q] = mine;
         gbase[q] = excl;
         s_rcv[q] = excl;
+        s_snd[q] = sent_excl;
     }
     __syncthreads();
     for (int r = warp; r < P; r += nwarps) {
+        write_list_flat(list_len, list_flat, r, s_snd[r]);
         int len = 0, e = -1;
         if (lane < G.nn[r]) {
             e = G.sender_of[r * kMaxNeighbors + lane];
@@ -1181,6 +1201,7 @@ struct StepTables {
     int* list_ret;
     int* list_len;
     int* send_base;
+    int* list_flat;
     int* gq;
     int* gbase;
     int* boff;
@@ -1220,6 +1241,7 @@ __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, 
                                                  const StepTables& T) {
     __shared__ int ws[33];
     __shared__ int s_rcv[kMaxRanks + 1];
+    __shared__ int s_snd[kMaxRanks];
     __shared__ int s_ts[kMaxRanks + 1];   // the current layout's tile starts, staged once
     const int P = G.P;
     const int t = threadIdx.x;
@@ -1289,19 +1311,28 @@ __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, 
             len = e >= 0 ? T.list_len[e] : 0;
         }
         const int sum = __reduce_add_sync(0xffffffffu, len);
-        if (lane == 0) s_rcv[q] = sum;
+        const int sent = lane < kMaxNeighbors ? T.list_len[q * kMaxNeighbors + lane] : 0;
+        const int out = __reduce_add_sync(0xffffffffu, sent);
+        if (lane == 0) {
+            s_rcv[q] = sum;
+            s_snd[q] = out;
+        }
     }
     __syncthreads();
     const int mine = t < P ? s_rcv[t] : 0;
-    int total_ghosts;
+    const int sent_all = t < P ? s_snd[t] : 0;
+    int total_ghosts, total_sent;
     const int gb = block_scan_excl<1024>(mine, total_ghosts, ws);
+    const int sb = block_scan_excl<1024>(sent_all, total_sent, ws);
     if (t < P) {
         T.gq[t] = mine;
         T.gbase[t] = gb;
         s_rcv[t] = gb;
+        s_snd[t] = sb;
     }
     __syncthreads();
     for (int q = warp; q < P; q += nwarps) {
+        write_list_flat(T.list_len, T.list_flat, q, s_snd[q]);
         int len = 0, e = -1;
         if (lane < G.nn[q]) {
             e = G.sender_of[q * kMaxNeighbors + lane];
@@ -2444,57 +2475,202 @@ __global__ void __launch_bounds__(NT, 3) k_step_move_staged(
     }
 }
 
+// ------------------------------------------------------- walks of the ghosts
+//
+// The refresh and the forward exchange gather one owner per ghost.  The owners
+// of one send list are sparse in the owned order (a face list holds about one
+// particle in 25), so a gather by ghost slot, receiver by receiver, reads the
+// 64-byte DRAM atoms of a sender's particles once for each of its lists, at
+// times too far apart for the cache.  The walk therefore goes sender by
+// sender and list by list (list_flat: where each list starts in that order):
+// all lists of a sender are in flight together, its particles come from DRAM
+// once and from L2 for the other lists, and the writes stay runs of
+// consecutive slots.  A warp takes up to four rows of 32 ghosts of that order
+// at a time, their loads in flight together; fewer where that spreads the
+// ghosts more evenly over the launch's warps and passes (a small plan is bound
+// by latency: one row on each of many warps hides more of it than four on a
+// few).
+constexpr int kWalkRows = 4;
+
+__device__ __forceinline__ int walk_height(int total, long long warps) {
+    const long long rows = (total + 32 * warps - 1) / (32 * warps);
+    const long long passes = (rows + kWalkRows - 1) / kWalkRows;
+    return passes < 1 ? 1 : static_cast<int>((rows + passes - 1) / passes);
+}
+
+// The largest e in [0, lists) with flat[e] <= t, by a whole warp (32 probes a
+// round; lists <= 26 * kMaxRanks < 32^3, flat[0] = 0).
+__device__ __forceinline__ int list_of(const int* __restrict__ flat, int lists, int t) {
+    const int lane = threadIdx.x & 31;
+    int e = 0;
+    for (int step = lists > 1024 ? 1024 : 32; step; step >>= 5) {
+        const int at = e + lane * step;
+        const unsigned below = __ballot_sync(0xffffffffu, at < lists && ro(flat + at) <= t);
+        e += (__popc(below) - 1) * step;
+    }
+    return e;
+}
+
+// Ghosts t0 + 32 u + lane of the walk, u < rows: their slots (-1 past the end
+// and in the rows not taken) and send lists.
+__device__ __forceinline__ void walk_rows(const int* __restrict__ flat,
+                                          const int* __restrict__ send_base, int lists, int t0,
+                                          int rows, int total, int (&slot)[kWalkRows],
+                                          int (&entry)[kWalkRows]) {
+    const int lane = threadIdx.x & 31;
+    const int e0 = list_of(flat, lists, t0);
+    const int end = min(t0 + 32 * rows, total);
+    // the next 32 lists' starts; `later` of them begin inside this chunk
+    const int start = e0 + 1 + lane < lists ? ro(flat + e0 + 1 + lane) : INT_MAX;
+    const int later = __popc(__ballot_sync(0xffffffffu, start < end));
+#pragma unroll
+    for (int u = 0; u < kWalkRows; ++u) entry[u] = e0;
+    for (int j = 0; j < later; ++j) {
+        const int first = __shfl_sync(0xffffffffu, start, j);
+#pragma unroll
+        for (int u = 0; u < kWalkRows; ++u) entry[u] += t0 + u * 32 + lane >= first;
+    }
+#pragma unroll
+    for (int u = 0; u < kWalkRows; ++u) {
+        const int t = t0 + u * 32 + lane;
+        if (later == 32) {   // more lists than one window (short or empty ones)
+            int lo = entry[u], hi = lists;   // flat[lo] <= t
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (ro(flat + mid) <= t) lo = mid;
+                else hi = mid;
+            }
+            entry[u] = lo;
+        }
+        slot[u] = t < end ? t - ro(flat + entry[u]) + ro(send_base + entry[u]) : -1;
+    }
+}
+
+// The same rows in slot order (receiver by receiver), `stride` apart.
+__device__ __forceinline__ void slot_rows(long long t0, long long stride, int rows, int total,
+                                          int (&slot)[kWalkRows]) {
+#pragma unroll
+    for (int u = 0; u < kWalkRows; ++u) {
+        const long long t = t0 + u * stride + (threadIdx.x & 31);
+        slot[u] = u < rows && t < total ? static_cast<int>(t) : -1;
+    }
+}
+
+// Words w0 + [0, N) of a field of `words` words a particle from owned particle
+// own[u] to ghost slot[u] (-1: none) in every row, all of them in flight.
+template <class W, int N>
+__device__ __forceinline__ void copy_words_rows(const W* from, W* to, int words,
+                                                const int (&own)[kWalkRows],
+                                                const int (&slot)[kWalkRows]) {
+    W v[kWalkRows][N];
+#pragma unroll
+    for (int u = 0; u < kWalkRows; ++u)
+#pragma unroll
+        for (int w = 0; w < N; ++w)
+            if (slot[u] >= 0) v[u][w] = ro(from + static_cast<long long>(own[u]) * words + w);
+#pragma unroll
+    for (int u = 0; u < kWalkRows; ++u)
+#pragma unroll
+        for (int w = 0; w < N; ++w)
+            if (slot[u] >= 0) to[static_cast<long long>(slot[u]) * words + w] = v[u][w];
+}
+
+template <int N, class W>
+__device__ __forceinline__ void copy_field_rows(const W* from, W* to, int words,
+                                                const int (&own)[kWalkRows],
+                                                const int (&slot)[kWalkRows]) {
+    int w0 = 0;
+#pragma unroll 1
+    for (; w0 + N <= words; w0 += N) copy_words_rows<W, N>(from + w0, to + w0, words, own, slot);
+#pragma unroll 1
+    for (; w0 < words; ++w0) copy_words_rows<W, 1>(from + w0, to + w0, words, own, slot);
+}
+
+// N words of every row at a time.
+template <int N>
+__device__ __forceinline__ void copy_rows(unsigned char* base, int bytes, long long owned_off,
+                                          long long ghost_off, const int (&own)[kWalkRows],
+                                          const int (&slot)[kWalkRows]) {
+    unsigned char* from = base + owned_off * bytes;
+    unsigned char* to = base + ghost_off * bytes;
+    if ((bytes & 7) == 0)
+        copy_field_rows<N>(reinterpret_cast<const unsigned long long*>(from),
+                        reinterpret_cast<unsigned long long*>(to), bytes >> 3, own, slot);
+    else
+        copy_field_rows<N>(reinterpret_cast<const unsigned*>(from), reinterpret_cast<unsigned*>(to),
+                        bytes >> 2, own, slot);
+}
+
 // Refresh along the existing plan (Host semantics, dsDecompX
 // src/halo.cpp:256-289 + 687): positions (+ shift) and velocities and every
 // registered field; forces of the ghosts become 0 again; mass, charge, type
-// and id keep the values of the plan build.  positions_only moves x, y, z.
-__global__ void __launch_bounds__(NT) k_halo_refresh(Grid G, Arrays A, long long owned_off,
-                                                     long long ghost_off, int positions_only,
-                                                     const int* info,
+// and id keep the values of the plan build.  POSITIONS moves x, y, z only.
+//
+// Bound by the DRAM atoms of the sparse owners and by L2 sectors.  Array by
+// array, four rows in flight: more arrays at once need registers that spill
+// (600 B of spills at four CTAs per SM: 590 against 370 us on the case below),
+// while 16 warps of twelve loads each already cover the latency.  Measured
+// (slot order before / list by list now): 16M clustered particles, 5.4M
+// ghosts, positions 158 / 136 us, 7 arrays 348 / 266 us; 13.6M particles, 11
+// arrays, 5.1M ghosts 772 / 371 us (585 us tile by tile).
+template <bool POSITIONS, bool BY_LIST>
+__global__ void __launch_bounds__(NT, POSITIONS ? 4 : 2) k_halo_refresh(Grid G, Arrays A, long long owned_off,
+                                                     long long ghost_off, const int* info,
+                                                     const int* __restrict__ list_flat,
+                                                     const int* __restrict__ send_base,
                                                      const int* __restrict__ ghost_owner,
                                                      const int* __restrict__ ghost_entry) {
     pdl_begin();
     if (*G.status & kStatusGhostOverflow) return;
     const int total = info[0];
-    // four ghosts per thread and pass: their owner indices, then their
-    // owners' positions, are all in flight before the first store (two per
-    // thread at 40 registers ran slower: 0.155 against 0.148 ms)
-    constexpr int U = 4;
-    const int step = gridDim.x * NT;
-    for (int s0 = blockIdx.x * NT + threadIdx.x; s0 < total; s0 += U * step) {
-        int own[U], ent[U];
+    const int lists = G.P * kMaxNeighbors;
+    const long long warps = static_cast<long long>(gridDim.x) * NW;
+    const int rows = walk_height(total, warps);
+    const long long stride = BY_LIST ? 32 : warps * 32;
+    for (long long t0 = (static_cast<long long>(blockIdx.x) * NW + (threadIdx.x >> 5)) * 32 *
+                        (BY_LIST ? rows : 1);
+         t0 < total; t0 += warps * 32 * rows) {
+        int slot[kWalkRows], entry[kWalkRows];
+        if constexpr (BY_LIST) {
+            walk_rows(list_flat, send_base, lists, static_cast<int>(t0), rows, total, slot, entry);
+        } else {
+            slot_rows(t0, stride, rows, total, slot);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int slot = s0 + u * step;
-            own[u] = slot < total ? ro(ghost_owner + slot) : 0;
-            ent[u] = slot < total ? ro(ghost_entry + slot) : 0;
+            for (int u = 0; u < kWalkRows; ++u)
+                entry[u] = slot[u] >= 0 ? ro(ghost_entry + slot[u]) : 0;
         }
-        double p[U][3];
+        int own[kWalkRows];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (s0 + u * step < total) {
-                const long long src = owned_off + own[u];
-                p[u][0] = A.d[0][src];
-                p[u][1] = A.d[1][src];
-                p[u][2] = A.d[2][src];
-            }
+        for (int u = 0; u < kWalkRows; ++u) own[u] = slot[u] >= 0 ? ro(ghost_owner + slot[u]) : 0;
+        double v[kWalkRows][3];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int slot = s0 + u * step;
-            if (slot >= total) continue;
-            const long long src = owned_off + own[u];
-            const double* sh = G.shift + 3ll * ent[u];
-            const long long gi = ghost_off + slot;
-            A.d[0][gi] = __dadd_rn(p[u][0], sh[0]);
-            A.d[1][gi] = __dadd_rn(p[u][1], sh[1]);
-            A.d[2][gi] = __dadd_rn(p[u][2], sh[2]);
-            A.d[6][gi] = 0.0; A.d[7][gi] = 0.0; A.d[8][gi] = 0.0;
-            if (!positions_only) {
-                A.d[3][gi] = A.d[3][src];
-                A.d[4][gi] = A.d[4][src];
-                A.d[5][gi] = A.d[5][src];
-                copy_fields(A.f, src, gi);
+        for (int u = 0; u < kWalkRows; ++u)
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                if (slot[u] >= 0) v[u][a] = ro(A.d[a] + owned_off + own[u]);
+#pragma unroll
+        for (int u = 0; u < kWalkRows; ++u) {
+            if (slot[u] < 0) continue;
+            const double* sh = G.shift + 3ll * entry[u];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                A.d[a][ghost_off + slot[u]] = __dadd_rn(v[u][a], ro(sh + a));
+                A.d[6 + a][ghost_off + slot[u]] = 0.0;
             }
+        }
+        if constexpr (!POSITIONS) {
+#pragma unroll
+            for (int u = 0; u < kWalkRows; ++u)
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    if (slot[u] >= 0) v[u][a] = ro(A.d[3 + a] + owned_off + own[u]);
+#pragma unroll
+            for (int u = 0; u < kWalkRows; ++u)
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    if (slot[u] >= 0) A.d[3 + a][ghost_off + slot[u]] = v[u][a];
+            for (int f = 0; f < A.f.count; ++f)
+                copy_rows<3>(A.f.base[f], A.f.bytes[f], owned_off, ghost_off, own, slot);
         }
     }
 }
@@ -2565,6 +2741,9 @@ __global__ void __launch_bounds__(NT) k_halo_refresh_owners(Grid G, Arrays A, lo
     }
 }
 
+// Forward exchange in slot order: one ghost per thread at full occupancy
+// (2M particles, 20 B a ghost: 12 us, and 26 against 25 us with a cold L2 for
+// the rows of the walk below, which holds a quarter of the warps).
 __global__ void __launch_bounds__(NT) k_forward_fields(Arrays A, long long owned_off,
                                                        long long ghost_off, FieldOps F,
                                                        const int* info,
@@ -2590,6 +2769,31 @@ __global__ void __launch_bounds__(NT) k_forward_fields(Arrays A, long long owned
                 for (int w = 0; w < (b >> 2); ++w) d[w] = s[w];
             }
         }
+    }
+}
+
+// Forward exchange list by list (walk_by_list): the owners' fields cross DRAM
+// once (16M particles, 20 B a ghost: 108 us in slot order, 74 us here).
+__global__ void __launch_bounds__(NT, 4) k_forward_by_list(Arrays A, long long owned_off,
+                                                           long long ghost_off, FieldOps F,
+                                                           int lists, const int* info,
+                                                           const int* __restrict__ list_flat,
+                                                           const int* __restrict__ send_base,
+                                                           const int* __restrict__ ghost_owner,
+                                                           const unsigned* status) {
+    pdl_begin();
+    if (*status & kStatusGhostOverflow) return;
+    const int total = info[0];
+    const long long warps = static_cast<long long>(gridDim.x) * NW;
+    const int rows = walk_height(total, warps);
+    for (long long t0 = (static_cast<long long>(blockIdx.x) * NW + (threadIdx.x >> 5)) * 32 * rows;
+         t0 < total; t0 += warps * 32 * rows) {
+        int slot[kWalkRows], entry[kWalkRows], own[kWalkRows];
+        walk_rows(list_flat, send_base, lists, static_cast<int>(t0), rows, total, slot, entry);
+#pragma unroll
+        for (int u = 0; u < kWalkRows; ++u) own[u] = slot[u] >= 0 ? ro(ghost_owner + slot[u]) : 0;
+        for (int t = 0; t < F.count; ++t)
+            copy_rows<2>(A.f.base[F.index[t]], A.f.bytes[F.index[t]], owned_off, ghost_off, own, slot);
     }
 }
 
@@ -2682,43 +2886,59 @@ __device__ __forceinline__ long long reduce_one<long long>(long long d, long lon
     }
 }
 
+// Components c, c + step, ... of owner's values (op)= those of its images: the
+// first image's slot is `first` (its value in flight with the owner's),
+// further ones bslot[k0 + 1, k1) in neighbor order.
 template <class T>
-__device__ __forceinline__ void reduce_images(unsigned char* base, int comps, int op, long long owner,
-                                              long long ghost_off, const int* bslot, int k0, int k1) {
+__device__ __forceinline__ void reduce_images(unsigned char* base, int comps, int op, int c, int step,
+                                              long long owner, long long ghost_off,
+                                              const int* __restrict__ bslot, int first, int k0,
+                                              int k1) {
     T* o = reinterpret_cast<T*>(base) + owner * comps;
-    for (int c = 0; c < comps; ++c) {
-        T acc = o[c];
-        for (int k = k0; k < k1; ++k)
-            acc = reduce_one<T>(acc, reinterpret_cast<const T*>(base)[(ghost_off + bslot[k]) * comps + c], op);
+    const T* ghosts = reinterpret_cast<const T*>(base) + ghost_off * comps;
+    for (; c < comps; c += step) {
+        T acc = reduce_one<T>(o[c], ro(ghosts + static_cast<long long>(first) * comps + c), op);
+        for (int k = k0 + 1; k < k1; ++k)
+            acc = reduce_one<T>(acc, ro(ghosts + static_cast<long long>(ro(bslot + k)) * comps + c), op);
         o[c] = acc;
     }
 }
 
+// One field per row of the grid.  A thread takes one component of one
+// boundary owner (up to three components of an owner sit on neighboring
+// threads, so a vector field is read and written in whole runs): the chain of
+// dependent loads is as short as it can be, and nothing waits for another
+// field.  Latency-bound while the fields fit the L2, DRAM-bound beyond: four
+// fields of 32 B, one owner with all its fields per thread before / now: 50k
+// particles 12.8 / 10.1 us, 2M 31 / 25, 8M 101 / 95, 16M 175 / 174.
 __global__ void __launch_bounds__(NT) k_reverse_fields(Arrays A, long long owned_off,
                                                        long long ghost_off, FieldOps F,
                                                        const int* info,
                                                        const int* __restrict__ bowner,
                                                        const int* __restrict__ boff,
                                                        const int* __restrict__ bslot,
+                                                       const int* __restrict__ bfirst,
                                                        const unsigned* status) {
     pdl_begin();
     if (*status & kStatusGhostOverflow) return;
-    const int B = info[1];
-    for (int b = blockIdx.x * NT + threadIdx.x; b < B; b += gridDim.x * NT) {
-        const long long owner = owned_off + bowner[b];
-        const int k0 = boff[b], k1 = boff[b + 1];
-        for (int t = 0; t < F.count; ++t) {
-            unsigned char* base = A.f.base[F.index[t]];
-            const int comps = F.components[t];
-            const int op = F.op[t];
-            switch (F.type[t]) {
-            case 0: reduce_images<int>(base, comps, op, owner, ghost_off, bslot, k0, k1); break;
-            case 1: reduce_images<long long>(base, comps, op, owner, ghost_off, bslot, k0, k1); break;
-            case 2: reduce_images<unsigned>(base, comps, op, owner, ghost_off, bslot, k0, k1); break;
-            case 3: reduce_images<unsigned long long>(base, comps, op, owner, ghost_off, bslot, k0, k1); break;
-            case 4: reduce_images<float>(base, comps, op, owner, ghost_off, bslot, k0, k1); break;
-            default: reduce_images<double>(base, comps, op, owner, ghost_off, bslot, k0, k1); break;
-            }
+    const int t = blockIdx.y;
+    unsigned char* base = A.f.base[F.index[t]];
+    const int comps = F.components[t];
+    const int op = F.op[t];
+    const unsigned step = comps < 3 ? comps : 3;
+    const unsigned items = static_cast<unsigned>(info[1]) * step;   // < 2^30 owners
+    for (unsigned w = blockIdx.x * NT + threadIdx.x; w < items; w += gridDim.x * NT) {
+        const unsigned b = step == 1 ? w : step == 2 ? w / 2u : w / 3u;
+        const int c = static_cast<int>(w - b * step);
+        const long long owner = owned_off + ro(bowner + b);
+        const int first = ro(bfirst + b), k0 = ro(boff + b), k1 = ro(boff + b + 1);
+        switch (F.type[t]) {
+        case 0: reduce_images<int>(base, comps, op, c, step, owner, ghost_off, bslot, first, k0, k1); break;
+        case 1: reduce_images<long long>(base, comps, op, c, step, owner, ghost_off, bslot, first, k0, k1); break;
+        case 2: reduce_images<unsigned>(base, comps, op, c, step, owner, ghost_off, bslot, first, k0, k1); break;
+        case 3: reduce_images<unsigned long long>(base, comps, op, c, step, owner, ghost_off, bslot, first, k0, k1); break;
+        case 4: reduce_images<float>(base, comps, op, c, step, owner, ghost_off, bslot, first, k0, k1); break;
+        default: reduce_images<double>(base, comps, op, c, step, owner, ghost_off, bslot, first, k0, k1); break;
         }
     }
 }
@@ -3228,13 +3448,13 @@ int sm_count() {
 // previous kernel on the stream drains, inside captured graphs too; errors
 // surface through cudaGetLastError like those of triple-chevron launches.
 template <class... Params, class... Args>
-void pdl_launch(void (*kernel)(Params...), int grid, int block, std::size_t smem, cudaStream_t s,
+void pdl_launch(void (*kernel)(Params...), dim3 grid, int block, std::size_t smem, cudaStream_t s,
                 Args&&... args) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(static_cast<unsigned>(grid));
+    config.gridDim = grid;
     config.blockDim = dim3(static_cast<unsigned>(block));
     config.dynamicSmemBytes = smem;
     config.stream = s;
@@ -3351,8 +3571,8 @@ void launch_halo_build(const Grid& G, const Arrays& A, long long owned_off, long
     if (S.marks) S.marks->mark(s, "halo_classify");
     pdl_launch(k_scan_counters, kHaloCounters, 1024, 0, s, S.cnt, S.pre, S.stride, G.tile_start + G.P);
     if (S.marks) S.marks->mark(s, "halo_scan");
-    pdl_launch(k_halo_layout, 1, 1024, 0, s, G, S.pre, S.stride, S.list_len, S.send_base, S.g, S.gbase,
-                                      S.boff, S.halo_info, S.cbase);
+    pdl_launch(k_halo_layout, 1, 1024, 0, s, G, S.pre, S.stride, S.list_len, S.send_base, S.list_flat,
+               S.g, S.gbase, S.boff, S.halo_info, S.cbase);
     if (S.marks) S.marks->mark(s, "halo_layout");
     // the tile's records staged in shared memory (all but the forces) when
     // they fit; plain launches keep the per-image reads
@@ -3427,7 +3647,7 @@ void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, con
 
 void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s) {
     StepTables T{S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.imm_base, S.emig_info,
-                 S.mig_results, S.list_ret, S.list_len, S.send_base, S.g, S.gbase, S.boff,
+                 S.mig_results, S.list_ret, S.list_len, S.send_base, S.list_flat, S.g, S.gbase, S.boff,
                  S.halo_info, S.cbase, S.cbase_imm, S.imm_tile_start, S.imm_tiles};
     pdl_launch(k_step_scan_layout, kStepCounters, 1024, 0, s, G, S.cnt, S.pre, S.stride, T, S.ticket);
     pdl_launch(k_tile_bases, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
@@ -3567,15 +3787,27 @@ int refresh_stage_bytes(const Arrays& A, bool positions_only) {
     return bytes;
 }
 
+// Bytes per particle that a full refresh copies.
+int refresh_bytes(const Arrays& A) {
+    int bytes = 48;
+    for (int f = 0; f < A.f.count; ++f) bytes += A.f.bytes[f];
+    return bytes;
+}
+
+// Whether a walk that copies `bytes` of every ghost's owner goes list by list:
+// once the owned arrays it reads exceed half of the L2 (126 MB).  Below that
+// the lists' repeated reads hit the L2 in any order and the list search only
+// costs.  Measured with a cold L2 and 30% boundary particles (slot order /
+// list by list): positions 2M (48 MB) 25.6 / 26.7 us, 4M (96 MB) 44 / 41, 8M
+// 80 / 63; full refresh of 92 B 0.3M (28 MB) 21.5 / 23.5, 1M (92 MB) 49 / 42,
+// 4M 168 / 107; forward of 20 B 2M (40 MB) 25.6 / 25.6, 4M (80 MB) 40 / 36,
+// 8M 75 / 54.
+bool walk_by_list(const Grid& G, int bytes) { return G.ncap * bytes > (64ll << 20); }
+
 void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, long long ghost_off,
                          bool positions_only, const Scratch& S, cudaStream_t s, int ctas_per_sm) {
     const int stage = refresh_stage_bytes(A, positions_only);
-    // the tile walk pays a fixed latency per tile, the ghost walk one sector
-    // per copied array and ghost: the tiles win once a full refresh copies
-    // nine arrays or more (measured: 11 arrays 1.19 against 1.50 ms, 7 arrays
-    // 0.39 against 0.31 ms, positions 0.30 against 0.15 ms)
-    const bool tiles = S.refresh_kind == 2 || (S.refresh_kind == 3 && !positions_only &&
-                                                6 + A.f.count >= 9);
+    const bool tiles = S.refresh_kind == 2;
     if (tiles && stage <= kStagedMaxBytes) {
         static bool attribute_set = false;   // once per process (one device per process)
         static std::mutex lock;
@@ -3616,18 +3848,30 @@ void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, lo
                                                   S.bfirst, S.ghost_entry);
         return;
     }
-    int grid = resident_grid(reinterpret_cast<const void*>(k_halo_refresh), G.gcap);
-    if (ctas_per_sm > 0 && grid > sm_count() * ctas_per_sm) grid = sm_count() * ctas_per_sm;
-    pdl_launch(k_halo_refresh, grid, NT, 0, s, G, A, owned_off, ghost_off,
-                                                      positions_only ? 1 : 0, S.halo_info,
-                                                      S.ghost_owner, S.ghost_entry);
+    auto walk = [&](auto kernel) {
+        int grid = resident_grid(reinterpret_cast<const void*>(kernel), G.gcap);
+        if (ctas_per_sm > 0 && grid > sm_count() * ctas_per_sm) grid = sm_count() * ctas_per_sm;
+        pdl_launch(kernel, grid, NT, 0, s, G, A, owned_off, ghost_off, S.halo_info, S.list_flat,
+                   S.send_base, S.ghost_owner, S.ghost_entry);
+    };
+    const bool by_list = S.refresh_kind == 3 && walk_by_list(G, positions_only ? 24 : refresh_bytes(A));
+    if (positions_only) by_list ? walk(k_halo_refresh<true, true>) : walk(k_halo_refresh<true, false>);
+    else by_list ? walk(k_halo_refresh<false, true>) : walk(k_halo_refresh<false, false>);
 }
 
 void launch_forward_fields(const Grid& G, const Arrays& A, long long owned_off,
                            long long ghost_off, const FieldOps& F, const Scratch& S,
                            cudaStream_t s) {
-    pdl_launch(k_forward_fields, resident_grid(reinterpret_cast<const void*>(k_forward_fields), G.gcap), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
-                                                        S.ghost_owner, G.status);
+    int bytes = 0;
+    for (int t = 0; t < F.count; ++t) bytes += A.f.bytes[F.index[t]];
+    if (walk_by_list(G, bytes)) {
+        pdl_launch(k_forward_by_list, resident_grid(reinterpret_cast<const void*>(k_forward_by_list), G.gcap),
+                   NT, 0, s, A, owned_off, ghost_off, F, G.P * kMaxNeighbors, S.halo_info,
+                   S.list_flat, S.send_base, S.ghost_owner, G.status);
+    } else {
+        pdl_launch(k_forward_fields, resident_grid(reinterpret_cast<const void*>(k_forward_fields), G.gcap), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
+                                                            S.ghost_owner, G.status);
+    }
 }
 
 void launch_reverse_sum3(const Grid& G, double* ox, double* oy, double* oz, const double* gx,
@@ -3652,8 +3896,8 @@ void launch_reverse_sum3(const Grid& G, double* ox, double* oy, double* oz, cons
 void launch_reverse_fields(const Grid& G, const Arrays& A, long long owned_off,
                            long long ghost_off, const FieldOps& F, const Scratch& S,
                            cudaStream_t s) {
-    pdl_launch(k_reverse_fields, resident_grid(reinterpret_cast<const void*>(k_reverse_fields), G.ncap), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
-                                                        S.bowner, S.boff, S.bslot, G.status);
+    pdl_launch(k_reverse_fields, dim3(resident_grid(reinterpret_cast<const void*>(k_reverse_fields), G.ncap), F.count), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
+                                                        S.bowner, S.boff, S.bslot, S.bfirst, G.status);
 }
 
 void launch_rebalance(const Grid& G, const double* work, RebalanceParams params,

@@ -45,6 +45,7 @@ struct Scratch {
     int* out_flags = nullptr;          // [P] out-of-domain flags
     int* list_len = nullptr;   // [P*26] send-list lengths
     int* send_base = nullptr;  // [P*26] first ghost slot of each send list
+    int* list_flat = nullptr;  // [P*26] first ghost of each send list, counted list by list
     int* g = nullptr;          // [P] ghosts per receiver
     int* gbase = nullptr;      // [P+1]
     int* ghost_owner = nullptr;  // [gcap] owned index of each ghost
@@ -79,9 +80,10 @@ struct Scratch {
     int classify_combine = 0;     // immigrant counters combined per warp before the atomics
     int move_staged = 1;          // 1: staged (one pass if it fits), 2: staged in passes,
                                   // 3: staged without forces, 0: direct reads
-    int refresh_kind = 3;         // refresh walk: 0 ghost by ghost, 1 owner by owner (the CSR),
-                                  // 2 tile by tile with the owners staged (when the stage fits),
-                                  // 3 tile by tile for a full refresh of 9 or more arrays, else 0
+    int refresh_kind = 3;         // refresh walk: 0 ghost by ghost in slot order, 1 owner by owner
+                                  // (the CSR), 2 tile by tile with the owners staged (when the
+                                  // stage fits), 3 ghost by ghost, sender by sender and list by
+                                  // list where the copied arrays exceed the L2, else as 0
     int reverse_per_sm = 0;       // CTAs per SM of the reverse sum; 0: one wave of the default shape
 };
 
