@@ -28,6 +28,8 @@ namespace dsx {
 
 // particles per tile of the tile kernels (256 threads x 2 groups of 32)
 constexpr int kTile = 512;
+// words of the step's per-tile bits (k_step_classify): 16 groups of 32 x 8
+constexpr int kTileBits = 128;
 constexpr int kMaxNeighbors = 26;
 constexpr int kMaxFields = 16;
 constexpr int kMaxRanks = 1024;
@@ -82,6 +84,7 @@ struct Grid {
     const double* shift = nullptr;       // [P*26*3]
     const signed char* dir = nullptr;    // [P*26*3]
     const unsigned* lut = nullptr;       // [P*64] halo flags -> neighbor mask
+    const unsigned char* need = nullptr; // [P*32] halo flags a list asks for, | 64 if it exists
     const int* coord = nullptr;          // [P] grid coordinates, 10 bits each (x<<20|y<<10|z)
 
     // geometry (changes with Dynamic boundaries)

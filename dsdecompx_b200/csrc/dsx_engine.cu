@@ -446,6 +446,8 @@ struct dsx_grid {
     signed char* d_dir = nullptr;
     unsigned* d_lut = nullptr;
     unsigned* d_lut_empty = nullptr;   // the same shape, every mask 0 (no halo)
+    unsigned char* d_need = nullptr;
+    unsigned char* d_need_empty = nullptr;   // no list exists
     int* d_coord = nullptr;
     // plain launches (per-call operations, one launch per subdomain)
     bool plain = false;
@@ -566,6 +568,7 @@ struct dsx_grid {
         G.shift = d_shift;
         G.dir = d_dir;
         G.lut = d_lut;
+        G.need = d_need;
         G.coord = d_coord;
         G.cuts = cuts;
         G.n = layout[cur][0];
@@ -655,6 +658,7 @@ struct dsx_grid {
         std::vector<double> shift(P * E * 3, 0.0);
         std::vector<signed char> dir(P * E * 3, 0);
         std::vector<unsigned> lut(static_cast<std::size_t>(P) * 64, 0u);
+        std::vector<unsigned char> need(static_cast<std::size_t>(P) * 32, 0);
         for (int s = 0; s < P; ++s) {
             const auto& list = topo[static_cast<std::size_t>(s)];
             nn[s] = static_cast<int>(list.size());
@@ -667,6 +671,11 @@ struct dsx_grid {
                 }
                 sender_of[idx] = sender_entry(s, static_cast<int>(n));
                 if (sender_of[idx] >= 0) recv_entry[sender_of[idx]] = idx;
+                // the comparisons this direction asks for (bits as `flags` below)
+                unsigned char& ask = need[static_cast<std::size_t>(s) * 32 + n];
+                if (list[n].rank >= 0) ask = 64;
+                for (int a = 0; a < 3 && ask; ++a)
+                    ask |= list[n].dir[a] < 0 ? 1u << (2 * a) : list[n].dir[a] > 0 ? 2u << (2 * a) : 0u;
             }
             // flags bit 2a: below lower+w on axis a; bit 2a+1: above upper-w
             for (unsigned flags = 1; flags < 64; ++flags) {
@@ -695,6 +704,8 @@ struct dsx_grid {
         d_dir = device_alloc<signed char>(fixed_owned, dir.size());
         d_lut = device_alloc<unsigned>(fixed_owned, lut.size());
         d_lut_empty = device_alloc<unsigned>(fixed_owned, lut.size());
+        d_need = device_alloc<unsigned char>(fixed_owned, need.size());
+        d_need_empty = device_alloc<unsigned char>(fixed_owned, need.size());
         std::vector<int> coord(static_cast<std::size_t>(P));
         for (int s = 0; s < P; ++s) {
             const auto& c = coords[static_cast<std::size_t>(s)];
@@ -704,6 +715,8 @@ struct dsx_grid {
         up(d_nn, nn); up(d_nbr, nbr); up(d_recv_entry, recv_entry); up(d_sender_of, sender_of);
         up(d_shift, shift); up(d_dir, dir); up(d_lut, lut); up(d_coord, coord);
         up(d_lut_empty, std::vector<unsigned>(lut.size(), 0u));
+        up(d_need, need);
+        up(d_need_empty, std::vector<unsigned char>(need.size(), 0));
 
         // uniform cuts (dsDecompX src/topology.cpp:63-75)
         std::vector<double> c;
@@ -761,9 +774,11 @@ struct dsx_grid {
         S.emig_info = device_alloc<int>(fixed_owned, 4);
         cuda_check(cudaMemset(S.emig_info, 0, 4 * sizeof(int)), "memset");
         S.mig_results = device_alloc<long long>(fixed_owned, static_cast<std::size_t>(P) * 6);
-        // per particle (per-call halo build) and per tile slot (batched step)
+        // halo masks per particle (per-call build, immigrants); bits and
+        // destinations per tile slot (batched step)
         const std::size_t slots = static_cast<std::size_t>(max_tiles) * dsx::kTile;
-        S.mask = device_alloc<unsigned>(fixed_owned, std::max<std::size_t>(slots, static_cast<std::size_t>(ncap)));
+        S.mask = device_alloc<unsigned>(fixed_owned, static_cast<std::size_t>(ncap));
+        S.bits = device_alloc<unsigned>(fixed_owned, static_cast<std::size_t>(max_tiles) * dsx::kTileBits);
         S.dest16 = device_alloc<unsigned short>(fixed_owned, slots);
         S.tile_bases = device_alloc<int>(fixed_owned, static_cast<std::size_t>(max_tiles) * 32);
         S.out_flags = device_alloc<int>(fixed_owned, P);
@@ -948,6 +963,7 @@ struct dsx_grid {
             // (the old layout's plan is dropped either way)
             dsx::Grid G = params();
             G.lut = d_lut_empty;
+            G.need = d_need_empty;
             dsx::launch_step_classify(G, A, owned_off(), S, stream);
             dsx::launch_step_layout(G, S, stream);
             dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);

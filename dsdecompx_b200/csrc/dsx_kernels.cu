@@ -644,34 +644,6 @@ __device__ __forceinline__ void count_group(unsigned m, int nn, int lane, int& a
     if (lane == kImageCounter) acc += total_images;
 }
 
-// count_group over K groups at once (lane holds one particle of each): the
-// same sums, one warp reduction per neighbor instead of one ballot per group.
-template <int K>
-__device__ __forceinline__ void count_groups(const unsigned (&m)[K], int lane, int& acc) {
-    unsigned all = 0;
-    int boundary = 0, images = 0;
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        all |= m[j];
-        boundary += m[j] != 0u;
-        images += __popc(m[j]);
-    }
-    const unsigned used = __reduce_or_sync(0xffffffffu, all);
-    if (!used) return;
-    for (unsigned rest = used; rest; rest &= rest - 1) {
-        const int n = __ffs(rest) - 1;
-        unsigned c = 0;
-#pragma unroll
-        for (int j = 0; j < K; ++j) c += (m[j] >> n) & 1u;
-        const int total = static_cast<int>(__reduce_add_sync(0xffffffffu, c));
-        if (lane == n) acc += total;
-    }
-    const int total_boundary = __reduce_add_sync(0xffffffffu, boundary);
-    const int total_images = __reduce_add_sync(0xffffffffu, images);
-    if (lane == kBoundaryCounter) acc += total_boundary;
-    if (lane == kImageCounter) acc += total_images;
-}
-
 // Immigrant totals of one 32-particle group: a lane with key >= 0 holds an
 // emigrant bound for subdomain `key` (-1: none) with the new owner's
 // neighbor mask `me`, counted into the owner's total, boundary, image and
@@ -1052,9 +1024,58 @@ __device__ __forceinline__ double wrap_if(const Grid& G, int a, double v) {
     return G.periodic[a] ? wrap_axis(v, G.lower[a], G.extent[a]) : v;
 }
 
-// F1: destination and new-owner halo mask of every owned particle; per-tile
-// counters; per-destination totals of the emigrants (atomics: only sums;
-// COMBINE: one per destination and warp, add_immigrants).
+// What the classify leaves of a tile, in words of 32 particles: a tile is 16
+// groups of 32, and a group has 8 words of one bit per particle -- the six
+// halo comparisons at the particle's (unchanged) owner (x below lower + w, x
+// above upper - w, y ..., z ...), "stays", and "leaves".  One byte per
+// particle instead of a 4-byte list mask and a 2-byte destination, and in the
+// form the counting wants: list n's members of a group are the AND of the (at
+// most three) comparison words its direction needs, so lane n forms them in
+// six logic operations for all 32 particles at once, where a mask per particle
+// cost one warp-wide pass per list in use.
+constexpr int kGroups = TILE / 32;
+constexpr int kGroupWords = 8;
+constexpr int kStayWord = 6;
+constexpr int kLeaveWord = 7;
+constexpr int kTileWords = kGroups * kGroupWords;
+static_assert(kTileWords == kTileBits, "engine allocation");
+
+// Lane n's list of subdomain s as masks over the six comparison words: `off`
+// is all ones where the list's direction does not ask for a comparison.
+struct ListTest {
+    unsigned off[6];
+    unsigned on;   // all ones for a list that exists
+};
+
+__device__ __forceinline__ ListTest list_test(const Grid& G, int s, int lane) {
+    const unsigned need = ro(G.need + s * 32 + lane);
+    ListTest t;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) t.off[k] = (need >> k) & 1u ? 0u : ~0u;
+    t.on = need & 64u ? ~0u : 0u;
+    return t;
+}
+
+__device__ __forceinline__ unsigned list_members(const ListTest& t, const unsigned (&w)[6]) {
+    unsigned h = t.on;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) h &= w[k] | t.off[k];
+    return h;
+}
+
+__device__ __forceinline__ unsigned halo_flags(const TileBounds& b, double px, double py, double pz) {
+    return (px < b.lo[0] ? 1u : 0u) | (px > b.hi[0] ? 2u : 0u) | (py < b.lo[1] ? 4u : 0u) |
+           (py > b.hi[1] ? 8u : 0u) | (pz < b.lo[2] ? 16u : 0u) | (pz > b.hi[2] ? 32u : 0u);
+}
+
+// F1: the bits of every owned particle (of the halo of its NEW owner where it
+// stays), destinations of those that leave, per-tile counters, and
+// per-destination totals of the leavers (atomics: only sums; COMBINE: one per
+// destination and warp, add_immigrants).
+//
+// Bound by reading the positions (24 B per particle): with the bits and the
+// lane-parallel counting a group of 32 costs about 70 warp instructions
+// against 220 with a mask and a destination per particle.
 template <int CT, int MINB, bool COMBINE>
 __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double* __restrict__ x,
                                                       const double* __restrict__ y,
@@ -1062,14 +1083,14 @@ __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double
                                                       int stride, int* imm_total, int* imm_list,
                                                       int* imm_bnd, int* imm_img,
                                                       unsigned short* __restrict__ dest_out,
-                                                      unsigned* __restrict__ mask_out,
+                                                      unsigned* __restrict__ bits_out,
                                                       int* pairs) {
     pdl_begin();
     constexpr int CI = TILE / CT;   // 32-particle groups per warp
     constexpr int CW = CT / 32;
     static_assert(CI * CT == TILE && CW >= 1, "tile split");
     __shared__ int s_cnt[CW][32];
-    __shared__ unsigned s_lut[64];   // the subdomain's halo flags -> neighbor mask
+    __shared__ __align__(16) unsigned s_bits[kTileWords];
     __shared__ unsigned short s_queue[TILE];   // tile slots left to the general path
     __shared__ int s_qn;
     const int g = blockIdx.x;
@@ -1092,37 +1113,32 @@ __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double
     }
     const TileBounds bs = halo_bounds(G, s);
     const Cell cell = cell_of(G, s);
-    for (int f = threadIdx.x; f < 64; f += CT) s_lut[f] = G.lut[s * 64 + f];
+    const ListTest list = list_test(G, s, lane);
     if (threadIdx.x == 0) s_qn = 0;
     __syncthreads();
-    const unsigned* lut = s_lut;
-    const int nn = G.nn[s];
     // with every periodic axis starting at 0, a coordinate inside its own
-    // cell needs no wrap arithmetic: both Host wraps return it (a -0 as +0)
-    const bool simple = (!G.periodic[0] || G.lower[0] == 0.0) &&
-                        (!G.periodic[1] || G.lower[1] == 0.0) &&
-                        (!G.periodic[2] || G.lower[2] == 0.0);
-    int acc = 0;
-    unsigned m[CI];
-    int fast = 0;   // this lane's particles that stay inside their own cell
+    // cell needs no wrap arithmetic: both Host wraps return it (a -0 as +0,
+    // which no comparison tells apart)
+    const bool simple = simple_wrap(G);
     const unsigned lt = lanemask_lt();
 #pragma unroll
     for (int j = 0; j < CI; ++j) {
         const int i = wbegin + j * 32 + lane;
         const bool valid = i < end;
-        const bool own = valid && simple && cell.lo[0] <= px[j] && px[j] < cell.hi[0] &&
-                         cell.lo[1] <= py[j] && py[j] < cell.hi[1] && cell.lo[2] <= pz[j] &&
-                         pz[j] < cell.hi[2];
-        m[j] = 0;
-        if (own) {
-            // stays: destination s, mask of the own subdomain
-            const double wx = G.periodic[0] && px[j] == 0.0 ? 0.0 : px[j];
-            const double wy = G.periodic[1] && py[j] == 0.0 ? 0.0 : py[j];
-            const double wz = G.periodic[2] && pz[j] == 0.0 ? 0.0 : pz[j];
-            m[j] = halo_mask(bs, lut, wx, wy, wz);
-            dest_out[static_cast<long long>(g) * TILE + (i - begin)] = static_cast<unsigned short>(s);
-            mask_out[static_cast<long long>(g) * TILE + (i - begin)] = m[j];
-            ++fast;
+        const bool own = valid && simple && inside_cell(cell, px[j], py[j], pz[j]);
+        uint4 a, b;
+        a.x = __ballot_sync(0xffffffffu, own && px[j] < bs.lo[0]);
+        a.y = __ballot_sync(0xffffffffu, own && px[j] > bs.hi[0]);
+        a.z = __ballot_sync(0xffffffffu, own && py[j] < bs.lo[1]);
+        a.w = __ballot_sync(0xffffffffu, own && py[j] > bs.hi[1]);
+        b.x = __ballot_sync(0xffffffffu, own && pz[j] < bs.lo[2]);
+        b.y = __ballot_sync(0xffffffffu, own && pz[j] > bs.hi[2]);
+        b.z = __ballot_sync(0xffffffffu, own);
+        b.w = 0u;
+        if (lane == 0) {
+            uint4* out = reinterpret_cast<uint4*>(s_bits + (warp * CI + j) * kGroupWords);
+            out[0] = a;
+            out[1] = b;
         }
         // every other particle of the tile waits in a queue for the
         // general path (one slot per particle; one shared atomic per group)
@@ -1134,28 +1150,28 @@ __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double
             if (valid && !own) s_queue[at + __popc(queued & lt)] = static_cast<unsigned short>(i - begin);
         }
     }
-    count_groups<CI>(m, lane, acc);
-    const int fast_stays = __reduce_add_sync(0xffffffffu, fast);
-    if (lane == kStepStay) acc += fast_stays;
     __syncthreads();
-    // The general path, 32 queued particles per warp and pass (a group with
-    // one leaver no longer runs it for all 32 lanes); it re-reads the
-    // positions, still in L1.
+    // The general path, 32 queued particles per warp and pass; it re-reads
+    // the positions, still in L1.
     const int nq = s_qn;
 #pragma unroll 1
     for (int q0 = warp * 32; q0 < nq; q0 += CW * 32) {
         const int q = q0 + lane;
-        const int i = q < nq ? begin + s_queue[q] : end;
+        const int l = q < nq ? s_queue[q] : TILE;
         int d = -1;
-        unsigned mg = 0, me = 0;
-        if (i < end) {
+        unsigned me = 0;
+        if (l < TILE) {
+            const int i = begin + l;
             double wx, wy, wz;
             d = destination_near(G, cell, ro(x + i), ro(y + i), ro(z + i), wx, wy, wz);
-            dest_out[static_cast<long long>(g) * TILE + (i - begin)] = static_cast<unsigned short>(d);
+            unsigned* word = s_bits + (l >> 5) * kGroupWords;
+            const unsigned bit = 1u << (l & 31);
             if (d == s) {
-                mg = halo_mask(bs, lut, wx, wy, wz);
-                mask_out[static_cast<long long>(g) * TILE + (i - begin)] = mg;
+                for (unsigned f = halo_flags(bs, wx, wy, wz) | 1u << kStayWord; f; f &= f - 1)
+                    atomicOr(word + __ffs(f) - 1, bit);
             } else {
+                atomicOr(word + kLeaveWord, bit);
+                dest_out[static_cast<long long>(g) * TILE + l] = static_cast<unsigned short>(d);
                 me = halo_mask(halo_bounds(G, d), G.lut + d * 64, wx, wy, wz);
                 // emigrants per (destination, source), for a sharded step
                 if (pairs) atomicAdd(&pairs[d * G.P + s], 1);
@@ -1172,13 +1188,29 @@ __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double
         }
         if constexpr (COMBINE)
             add_immigrants(d >= 0 && d != s ? d : -1, me, lane, imm_total, imm_bnd, imm_img, imm_list);
-        count_group(mg, nn, lane, acc);
-        const int stays = __popc(__ballot_sync(0xffffffffu, d == s));
-        const int emigs = __popc(__ballot_sync(0xffffffffu, d >= 0 && d != s));
-        if (lane == kStepStay) acc += stays;
-        if (lane == kStepEmig) acc += emigs;
     }
+    if (nq) __syncthreads();   // uniform: the general path changed the words
+    // counters: lane n of a warp its list over the warp's groups
+    int acc = 0, boundary = 0, stays = 0, emigs = 0;
+#pragma unroll
+    for (int j = 0; j < CI; ++j) {
+        const uint4* in = reinterpret_cast<const uint4*>(s_bits + (warp * CI + j) * kGroupWords);
+        const uint4 a = in[0], b = in[1];
+        const unsigned w[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+        const unsigned members = list_members(list, w);
+        acc += __popc(members);
+        boundary += __popc(__reduce_or_sync(0xffffffffu, members));
+        stays += __popc(b.z);
+        emigs += __popc(b.w);
+    }
+    const int images = __reduce_add_sync(0xffffffffu, acc);   // lanes without a list hold 0
+    if (lane == kBoundaryCounter) acc = boundary;
+    if (lane == kImageCounter) acc = images;
+    if (lane == kStepStay) acc = stays;
+    if (lane == kStepEmig) acc = emigs;
     s_cnt[warp][lane] = acc;
+    for (int k = threadIdx.x; k < kTileWords; k += CT)
+        bits_out[static_cast<long long>(g) * kTileWords + k] = s_bits[k];
     __syncthreads();
     if (threadIdx.x < kStepCounters) {
         int sum = 0;
@@ -1393,163 +1425,208 @@ __device__ __forceinline__ void write_ghost_wrapped(const Grid& G, const Arrays&
     copy_fields(A.f, src, gi);
 }
 
+// Shared memory of a move's index phase.
+struct MoveIndex {
+    int cnt[NW][32];
+    int base[32];                        // the tile's first entry of each counter
+    int off[kMaxNeighbors + 1];          // where each list starts in `own`
+    unsigned short own[kStageCap];       // ghost images list by list: tile slot | list << 9
+    int ni[TILE];                        // new owned index of the stays
+};
+
+struct MoveOutputs {
+    int* ghost_owner;
+    int* ghost_entry;
+    int* bowner;
+    int* boff;
+    int* bslot;
+    int* bfirst;
+};
+
+// The index phase of a move, from the tile's bits alone (it runs while the
+// record copies land): new slots of the stays, boundary owners with their
+// image slots (in neighbor order), and the ghost images listed list by list
+// in shared memory (a tile with more images than the list holds, only
+// possible with a halo wider than half a cell, is not `staged`).  `word`: lane
+// l < 16's word of the warp's two groups.  Ends without a barrier.
+struct MoveTile {
+    unsigned members[ITEMS];   // lane n: members of list n
+    unsigned mask[ITEMS];      // lists of this lane's particle
+    int ni[ITEMS];             // new slot of this lane's particle (a stay), else -1
+    int run0;                  // lane k: the warp's first entry of counter k
+    int Q;                     // ghost images of the tile
+    bool staged;
+};
+
+__device__ __forceinline__ MoveTile index_move(const Grid& G, int s, unsigned word, int base,
+                                               bool ghosts, int index_outputs, MoveIndex& S,
+                                               const MoveOutputs& O) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lt = lanemask_lt();
+    const ListTest list = list_test(G, s, lane);
+    MoveTile t;
+    unsigned any[ITEMS], stay[ITEMS];
+    int acc = 0, stays = 0, boundary = 0;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        unsigned w[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) w[k] = __shfl_sync(0xffffffffu, word, j * kGroupWords + k);
+        stay[j] = __shfl_sync(0xffffffffu, word, j * kGroupWords + kStayWord);
+        t.members[j] = ghosts ? list_members(list, w) : 0u;
+        any[j] = __reduce_or_sync(0xffffffffu, t.members[j]);
+        acc += __popc(t.members[j]);
+        stays += __popc(stay[j]);
+        boundary += __popc(any[j]);
+        t.mask[j] = 0;
+        if ((any[j] >> lane) & 1u) {
+            unsigned flags = 0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) flags |= ((w[k] >> lane) & 1u) << k;
+            t.mask[j] = ro(G.lut + s * 64 + flags);
+        }
+    }
+    const int images = __reduce_add_sync(0xffffffffu, acc);
+    S.cnt[warp][lane] = lane == kBoundaryCounter ? boundary
+                        : lane == kImageCounter  ? images
+                        : lane == kStepStay      ? stays
+                                                 : acc;
+    if (threadIdx.x < kStepCounters) S.base[threadIdx.x] = base;
+    __syncthreads();
+    // every counter's total over the warps and the part before this warp;
+    // then the lists' places in the staging list (an exclusive scan)
+    int tot = 0, before = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        const int c = S.cnt[w][lane];
+        tot += c;
+        before += w < warp ? c : 0;
+    }
+    const int mine = lane < kMaxNeighbors ? tot : 0;
+    const int incl = warp_inclusive_sum(mine);
+    t.Q = __shfl_sync(0xffffffffu, incl, 31);
+    if (warp == 0 && lane <= kMaxNeighbors) S.off[lane] = incl - mine;
+    t.staged = t.Q <= kStageCap;
+    int run = (lane < kStepCounters ? S.base[lane] : 0) + before;
+    int lrun = incl - mine + before;
+    t.run0 = run;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int l = (warp * ITEMS + j) * 32 + lane;
+        const int ni = __shfl_sync(0xffffffffu, run, kStepStay) + __popc(stay[j] & lt);
+        t.ni[j] = (stay[j] >> lane) & 1u ? ni : -1;
+        if (t.ni[j] >= 0) S.ni[l] = ni;
+        if (any[j]) {
+            const int b = __shfl_sync(0xffffffffu, run, kBoundaryCounter) + __popc(any[j] & lt);
+            const int pm = __popc(t.mask[j]);
+            const int pincl = warp_inclusive_sum(pm);
+            int img = __shfl_sync(0xffffffffu, run, kImageCounter) + pincl - pm;
+            if (pm && index_outputs) {
+                O.bowner[b] = ni;
+                O.boff[b] = img;
+            }
+            // image by image of every particle at once: list n's members and
+            // running slots come from lane n
+            bool first = true;
+            unsigned m = t.mask[j];
+            while (__any_sync(0xffffffffu, m != 0)) {
+                const int n = m ? __ffs(m) - 1 : 0;
+                const unsigned members = __shfl_sync(0xffffffffu, t.members[j], n);
+                const int slot = __shfl_sync(0xffffffffu, run, n) + __popc(members & lt);
+                const int at = __shfl_sync(0xffffffffu, lrun, n) + __popc(members & lt);
+                if (m) {
+                    if (index_outputs) {
+                        O.bslot[img] = slot;
+                        if (first) O.bfirst[b] = slot;
+                    }
+                    if (t.staged) S.own[at] = static_cast<unsigned short>(l | n << 9);
+                    ++img;
+                    first = false;
+                    m &= m - 1;
+                }
+            }
+            const int c = __popc(t.members[j]);
+            const int group_images = __shfl_sync(0xffffffffu, pincl, 31);
+            if (lane < kMaxNeighbors) {
+                run += c;
+                lrun += c;
+            }
+            if (lane == kBoundaryCounter) run += __popc(any[j]);
+            if (lane == kImageCounter) run += group_images;
+        }
+        if (lane == kStepStay) run += __popc(stay[j]);
+    }
+    return t;
+}
+
+// Ghost images of a tile, write(list, slot, tile slot): from the staging list
+// (consecutive threads on consecutive slots of a list; after a barrier), or
+// from the hitting lanes of a tile that is not staged.
+template <class W>
+__device__ __forceinline__ void each_image(const MoveTile& t, const MoveIndex& S, W&& write) {
+    if (t.staged) {
+        for (int q = threadIdx.x; q < t.Q; q += NT) {
+            const int e = S.own[q];
+            const int n = e >> 9;
+            write(n, S.base[n] + (q - S.off[n]), e & (TILE - 1));
+        }
+        return;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lt = lanemask_lt();
+    int run = t.run0;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        unsigned m = t.mask[j];
+        while (__any_sync(0xffffffffu, m != 0)) {
+            const int n = m ? __ffs(m) - 1 : 0;
+            const unsigned members = __shfl_sync(0xffffffffu, t.members[j], n);
+            const int slot = __shfl_sync(0xffffffffu, run, n) + __popc(members & lt);
+            if (m) {
+                write(n, slot, (warp * ITEMS + j) * 32 + lane);
+                m &= m - 1;
+            }
+        }
+        run += __popc(t.members[j]);
+    }
+}
+
 // F4: retained particles move to their new slots (stable) and write their
-// ghost images (staged per tile, then written list by list with coalesced
-// stores); emigrants are listed for the multi-split.  On a ghost overflow the
-// move still completes (the engine grows the ghost region and rebuilds).
+// ghost images.  On a ghost overflow the move still completes (the engine
+// grows the ghost region and rebuilds).  This form reads HBM directly (a
+// record too wide to stage).
 __global__ void __launch_bounds__(NT, 4) k_step_move(Grid G, Arrays A, long long src_off,
                                                   long long dst_off, long long ghost_off,
-                                                  const int* pre, int stride, const int* cbase_ret,
-                                                  const unsigned short* __restrict__ dest_in,
-                                                  const unsigned* __restrict__ mask_in,
-                                                  int* emig_src, int* emig_dst, int* ghost_owner,
-                                                  int* ghost_entry, int* bowner, int* boff,
-                                                  int* bslot, int* bfirst) {
+                                                  const unsigned* __restrict__ bits,
+                                                  const int* __restrict__ tile_bases,
+                                                  MoveOutputs O) {
     pdl_begin();
-    __shared__ int s_cnt[NW][32];
-    __shared__ int s_base[32];
-    __shared__ int s_off[kMaxNeighbors + 1];
-    __shared__ unsigned short s_own[kStageCap];
-    __shared__ int s_ni[TILE];
+    __shared__ MoveIndex S;
     const int g = blockIdx.x;
     if (g >= G.tile_start[G.P]) return;
     const bool ghosts = !(*G.status & kStatusGhostOverflow);
     const int4 td = G.tiles[g];
-    const int s = td.x, begin = td.y, end = td.z, first = td.w;
+    const int s = td.x, begin = td.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wbegin = begin + warp * 32 * ITEMS;
-    const int nn = G.nn[s];
-    const unsigned lt = lanemask_lt();
-
-    int dest[ITEMS];
-    unsigned msk[ITEMS];
-    int acc = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int i = wbegin + j * 32 + lane;
-        dest[j] = -1;
-        msk[j] = 0;
-        if (i < end) {
-            dest[j] = dest_in[static_cast<long long>(g) * TILE + (i - begin)];
-            if (dest[j] == s) msk[j] = mask_in[static_cast<long long>(g) * TILE + (i - begin)];
-        }
-        count_group(msk[j], nn, lane, acc);
-        const int stays = __popc(__ballot_sync(0xffffffffu, dest[j] == s));
-        const int emigs = __popc(__ballot_sync(0xffffffffu, dest[j] >= 0 && dest[j] != s));
-        if (lane == kStepStay) acc += stays;
-        if (lane == kStepEmig) acc += emigs;
-    }
-    s_cnt[warp][lane] = acc;
-    if (threadIdx.x < kStepCounters) {
-        const int k = threadIdx.x;
-        int base;
-        if (k < kHaloCounters) base = cbase_ret[s * kHaloCounters + k] + pre[k * stride + g] - pre[k * stride + first];
-        else if (k == kStepStay) base = G.obase_next[s] + pre[k * stride + g] - pre[k * stride + first];
-        else base = pre[k * stride + g];
-        s_base[k] = base;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // staging offsets of the lists: lane n sums its list over the warps,
-        // then an exclusive scan over the lanes
-        int tot = 0;
-        if (lane < nn)
-            for (int w = 0; w < NW; ++w) tot += s_cnt[w][lane];
-        const int incl = warp_inclusive_sum(tot);
-        if (lane < nn) s_off[lane] = incl - tot;
-        if (lane == 31) s_off[nn] = incl;
-    }
-    __syncthreads();
-    const int Q = s_off[nn];
-    const bool staged = Q <= kStageCap;
-    int run = 0, lrun = 0;
-    if (lane < kStepCounters) {
-        run = s_base[lane];
-        if (lane < nn) lrun = s_off[lane];
-        for (int w = 0; w < warp; ++w) {
-            run += s_cnt[w][lane];
-            lrun += s_cnt[w][lane];
-        }
-    }
+    const unsigned word = lane < ITEMS * kGroupWords
+        ? ro(bits + static_cast<long long>(g) * kTileWords + warp * ITEMS * kGroupWords + lane) : 0u;
+    const int base = threadIdx.x < kStepCounters ? tile_bases[static_cast<long long>(g) * 32 + threadIdx.x] : 0;
+    const MoveTile t = index_move(G, s, word, base, ghosts, 1, S, O);
     const double* shift = G.shift + static_cast<long long>(s) * kMaxNeighbors * 3;
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-        const int i = wbegin + j * 32 + lane;
-        const bool stay = dest[j] == s;
-        const bool emig = dest[j] >= 0 && !stay;
-        const unsigned bs_ = __ballot_sync(0xffffffffu, stay);
-        const unsigned be = __ballot_sync(0xffffffffu, emig);
-        const int ni = __shfl_sync(0xffffffffu, run, kStepStay) + __popc(bs_ & lt);
-        const int eb = __shfl_sync(0xffffffffu, run, kStepEmig) + __popc(be & lt);
-        if (stay) {
-            const long long src = src_off + i;
-            move_record(A, src, dst_off + ni, wrap_if(G, 0, ro(A.d[0] + src)),
-                        wrap_if(G, 1, ro(A.d[1] + src)), wrap_if(G, 2, ro(A.d[2] + src)));
-            s_ni[i - begin] = ni;
-        } else if (emig) {
-            emig_src[eb] = i;
-            emig_dst[eb] = dest[j];
-        }
-        const unsigned mj = ghosts ? msk[j] : 0u;
-        const unsigned any = __ballot_sync(0xffffffffu, mj != 0);
-        if (any) {
-            const int b = __shfl_sync(0xffffffffu, run, kBoundaryCounter) + __popc(any & lt);
-            const int pm = __popc(mj);
-            const int incl = warp_inclusive_sum(pm);
-            const int img = __shfl_sync(0xffffffffu, run, kImageCounter) + incl - pm;
-            if (mj) {
-                bowner[b] = ni;
-                boff[b] = img;
-            }
-            int k = 0;
-            const unsigned used = __reduce_or_sync(0xffffffffu, mj);
-            for (unsigned rest = used; rest; rest &= rest - 1) {
-                const int n = __ffs(rest) - 1;
-                const unsigned hit = __ballot_sync(0xffffffffu, (mj >> n) & 1u);
-                const int list_base = __shfl_sync(0xffffffffu, run, n);
-                const int stage_base = __shfl_sync(0xffffffffu, lrun, n);
-                if ((mj >> n) & 1u) {
-                    const int rank = __popc(hit & lt);
-                    const int slot = list_base + rank;
-                    bslot[img + k] = slot;
-                    if (k == 0) bfirst[b] = slot;
-                    ++k;
-                    if (staged) {
-                        s_own[stage_base + rank] = static_cast<unsigned short>(i - begin);
-                    } else {
-                        write_ghost_wrapped(G, A, src_off + i, ghost_off + slot, shift + 3 * n);
-                        ghost_owner[slot] = ni;
-                        ghost_entry[slot] = s * kMaxNeighbors + n;
-                    }
-                }
-                if (lane == n) {
-                    run += __popc(hit);
-                    lrun += __popc(hit);
-                }
-            }
-            const int group_images = __shfl_sync(0xffffffffu, incl, 31);
-            if (lane == kBoundaryCounter) run += __popc(any);
-            if (lane == kImageCounter) run += group_images;
-        }
-        if (lane == kStepStay) run += __popc(bs_);
-        if (lane == kStepEmig) run += __popc(be);
+        if (t.ni[j] < 0) continue;
+        const long long src = src_off + begin + (warp * ITEMS + j) * 32 + lane;
+        move_record(A, src, dst_off + t.ni[j], wrap_if(G, 0, ro(A.d[0] + src)),
+                    wrap_if(G, 1, ro(A.d[1] + src)), wrap_if(G, 2, ro(A.d[2] + src)));
     }
-    if (!ghosts || !staged) return;
+    if (!ghosts) return;
     __syncthreads();
-    for (int q = threadIdx.x; q < Q; q += NT) {
-        int lo = 0, hi = nn;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (s_off[mid] <= q) lo = mid;
-            else hi = mid;
-        }
-        const int n = lo;
-        const int slot = s_base[n] + (q - s_off[n]);
-        const int l = s_own[q];
+    each_image(t, S, [&](int n, int slot, int l) {
         write_ghost_wrapped(G, A, src_off + begin + l, ghost_off + slot, shift + 3 * n);
-        ghost_owner[slot] = s_ni[l];
-        ghost_entry[slot] = s * kMaxNeighbors + n;
-    }
+        O.ghost_owner[slot] = S.ni[l];
+        O.ghost_entry[slot] = s * kMaxNeighbors + n;
+    });
 }
 
 // ------------------------------------------------------------ bulk staging
@@ -2175,19 +2252,40 @@ __device__ __forceinline__ void fill_tiles_grid(int P, int tile, const int* n, c
 }
 
 // Counter bases of every tile of the layout (30 per tile, row stride 32), so
-// that the move reads them with one load per tile; and the tile descriptors
-// of the next layout and of its immigrant segments (imm_in: immigrants per
-// subdomain, imm_base: where they start, imm_ts: their tile starts).
+// that the move reads them with one load per tile; the list of emigrants, in
+// (source subdomain, source order); and the tile descriptors of the next
+// layout and of its immigrant segments (imm_in: immigrants per subdomain,
+// imm_base: where they start, imm_ts: their tile starts).  A warp per tile.
 __global__ void __launch_bounds__(NT) k_tile_bases(Grid G, const int* pre, int stride,
                                                    const int* cbase_ret, int* tile_bases,
+                                                   const unsigned* __restrict__ bits,
+                                                   const unsigned short* __restrict__ dest,
+                                                   int* emig_src, int* emig_dst,
                                                    const int* imm_in, const int* imm_base,
                                                    const int* imm_ts, int4* imm_tiles) {
     pdl_begin();
     const int ntiles = G.tile_start[G.P];
-    for (long long idx = blockIdx.x * static_cast<long long>(NT) + threadIdx.x;
-         idx < static_cast<long long>(ntiles) * 32; idx += static_cast<long long>(gridDim.x) * NT) {
-        const int g = static_cast<int>(idx >> 5), k = static_cast<int>(idx & 31);
-        if (k < kStepCounters) tile_bases[idx] = tile_base(G, pre, stride, cbase_ret, g, G.tiles[g], k);
+    const int lane = threadIdx.x & 31;
+    for (int g = blockIdx.x * NW + (threadIdx.x >> 5); g < ntiles; g += gridDim.x * NW) {
+        const int4 td = G.tiles[g];
+        const long long slot0 = static_cast<long long>(g) * TILE + lane * 32;
+        unsigned leave = lane < kGroups
+            ? ro(bits + static_cast<long long>(g) * kTileWords + lane * kGroupWords + kLeaveWord) : 0u;
+        int first = 0;
+        if (lane < kStepCounters) {
+            first = tile_base(G, pre, stride, cbase_ret, g, td, lane);
+            tile_bases[static_cast<long long>(g) * 32 + lane] = first;
+        }
+        const int emigrants = __shfl_sync(0xffffffffu, first, kStepEmig);
+        if (__any_sync(0xffffffffu, leave != 0)) {
+            const int c = __popc(leave);
+            int e = emigrants + warp_inclusive_sum(c) - c;
+            for (; leave; leave &= leave - 1, ++e) {
+                const int l = __ffs(leave) - 1;
+                emig_src[e] = td.y + lane * 32 + l;
+                emig_dst[e] = dest[slot0 + l];
+            }
+        }
     }
     fill_tiles_grid(G.P, G.tile, G.n_next, G.obase_next, G.tile_start_next, G.tiles_next);
     fill_tiles_grid(G.P, G.tile, imm_in, imm_base, imm_ts, imm_tiles);
@@ -2228,38 +2326,25 @@ __global__ void __launch_bounds__(1024) k_step_export(Grid G, const int* pre, in
 // and masks, and only the pass with index_outputs writes its results.
 template <bool FULL, bool DIRECT_FORCES>
 __global__ void __launch_bounds__(NT, 3) k_step_move_staged(
-    Grid G, Arrays A, long long src_off, long long dst_off, long long ghost_off, const int* pre,
-    int stride, const int* cbase_ret, const unsigned short* __restrict__ dest_in,
-    const unsigned* __restrict__ mask_in, const int* __restrict__ tile_bases, int* emig_src,
-    int* emig_dst, int* ghost_owner, int* ghost_entry, int* bowner, int* boff, int* bslot, int* bfirst, int a0,
+    Grid G, Arrays A, long long src_off, long long dst_off, long long ghost_off,
+    const unsigned* __restrict__ bits, const int* __restrict__ tile_bases, MoveOutputs O, int a0,
     int a1, int index_outputs) {
     pdl_begin();
     extern __shared__ __align__(16) unsigned char s_rec[];
     __shared__ __align__(8) unsigned long long s_bar;
     __shared__ int s_seg[kStagedArrays];
-    __shared__ int s_cnt[NW][32];
-    __shared__ int s_base[32];
-    __shared__ int s_off[kMaxNeighbors + 1];
-    __shared__ unsigned short s_own[kStageCap];
-    __shared__ int s_ni[TILE];
+    __shared__ MoveIndex S;
     const int g = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // destinations, masks (per tile slot) and the counter bases (per tile)
-    // need only the tile index: they are read together with the descriptor
+    // the bits and the counter bases need only the tile index: they are read
+    // together with the descriptor
     const int4 td = G.tiles[g];
-    const long long slot0 = static_cast<long long>(g) * TILE + warp * 32 * ITEMS + lane;
-    unsigned short d16[ITEMS];
-    unsigned mraw[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        d16[j] = dest_in[slot0 + j * 32];
-        mraw[j] = mask_in[slot0 + j * 32];
-    }
+    const unsigned word = lane < ITEMS * kGroupWords
+        ? ro(bits + static_cast<long long>(g) * kTileWords + warp * ITEMS * kGroupWords + lane) : 0u;
     const int base = threadIdx.x < kStepCounters ? tile_bases[static_cast<long long>(g) * 32 + threadIdx.x] : 0;
     if (g >= G.tile_start[G.P]) return;
     const int s = td.x, begin = td.y, end = td.z;
     const unsigned bar = smem_u32(&s_bar);
-    const int wbegin = begin + warp * 32 * ITEMS;
     // the tile's records go out as soon as the descriptor is known
     if (warp == 0) {
         if (lane == 0) {
@@ -2269,122 +2354,15 @@ __global__ void __launch_bounds__(NT, 3) k_step_move_staged(
         __syncwarp();
         stage_issue(A, src_off, begin, end, s_rec, bar, s_seg, lane, a0, a1, DIRECT_FORCES);
     }
-    // (slots past the tile's end hold stale values: masked here; the mask
-    // is only meaningful for a stay)
-    int dest[ITEMS];
-    unsigned msk[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const bool in = wbegin + j * 32 + lane < end;
-        dest[j] = in ? static_cast<int>(d16[j]) : -1;
-        msk[j] = in ? mraw[j] : 0u;
-    }
     const bool ghosts = !(*G.status & kStatusGhostOverflow);
-    const int nn = G.nn[s];
-    const unsigned lt = lanemask_lt();
-    int acc = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        if (dest[j] != s) msk[j] = 0;
-        count_group(msk[j], nn, lane, acc);
-        const int stays = __popc(__ballot_sync(0xffffffffu, dest[j] == s));
-        const int emigs = __popc(__ballot_sync(0xffffffffu, dest[j] >= 0 && dest[j] != s));
-        if (lane == kStepStay) acc += stays;
-        if (lane == kStepEmig) acc += emigs;
-    }
-    s_cnt[warp][lane] = acc;
-    if (threadIdx.x < kStepCounters) s_base[threadIdx.x] = base;
-    __syncthreads();
-    // staging offsets of the lists: lane n sums its list over the warps, then
-    // an exclusive scan over the lanes (every warp computes them; warp 0
-    // keeps them for the ghost pass)
-    int tot = 0;
-    if (lane < nn)
-        for (int w = 0; w < NW; ++w) tot += s_cnt[w][lane];
-    const int sincl = warp_inclusive_sum(tot);
-    const int Q = __shfl_sync(0xffffffffu, sincl, 31);
-    if (warp == 0) {
-        if (lane < nn) s_off[lane] = sincl - tot;
-        if (lane == 31) s_off[nn] = sincl;
-    }
-    const bool staged = Q <= kStageCap;
-    int run = 0, lrun = 0;
-    if (lane < kStepCounters) {
-        run = s_base[lane];
-        if (lane < nn) lrun = sincl - tot;
-        for (int w = 0; w < warp; ++w) {
-            run += s_cnt[w][lane];
-            lrun += s_cnt[w][lane];
-        }
-    }
-    const int run0 = run;
-    // the index work needs only destinations and masks, so it runs while the
-    // record copies are still landing: new slots, emigrant list, boundary
-    // owners and their image slots, and the ghost images staged by list
-    int nis[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int i = wbegin + j * 32 + lane;
-        const int l = i - begin;
-        const bool stay = dest[j] == s;
-        const bool emig = dest[j] >= 0 && !stay;
-        const unsigned bs_ = __ballot_sync(0xffffffffu, stay);
-        const unsigned be = __ballot_sync(0xffffffffu, emig);
-        const int ni = __shfl_sync(0xffffffffu, run, kStepStay) + __popc(bs_ & lt);
-        const int eb = __shfl_sync(0xffffffffu, run, kStepEmig) + __popc(be & lt);
-        nis[j] = ni;
-        if (stay) {
-            s_ni[l] = ni;
-        } else if (emig && index_outputs) {
-            emig_src[eb] = i;
-            emig_dst[eb] = dest[j];
-        }
-        const unsigned mj = ghosts ? msk[j] : 0u;
-        const unsigned any = __ballot_sync(0xffffffffu, mj != 0);
-        if (any) {
-            const int b = __shfl_sync(0xffffffffu, run, kBoundaryCounter) + __popc(any & lt);
-            const int pm = __popc(mj);
-            const int incl = warp_inclusive_sum(pm);
-            const int img = __shfl_sync(0xffffffffu, run, kImageCounter) + incl - pm;
-            if (mj && index_outputs) {
-                bowner[b] = ni;
-                boff[b] = img;
-            }
-            int k = 0;
-            const unsigned used = __reduce_or_sync(0xffffffffu, mj);
-            for (unsigned rest = used; rest; rest &= rest - 1) {
-                const int n = __ffs(rest) - 1;
-                const unsigned hit = __ballot_sync(0xffffffffu, (mj >> n) & 1u);
-                const int list_base = __shfl_sync(0xffffffffu, run, n);
-                const int stage_base = __shfl_sync(0xffffffffu, lrun, n);
-                if ((mj >> n) & 1u) {
-                    const int rank = __popc(hit & lt);
-                    if (index_outputs) {
-                        bslot[img + k] = list_base + rank;
-                        if (k == 0) bfirst[b] = list_base + rank;
-                    }
-                    ++k;
-                    if (staged) s_own[stage_base + rank] = static_cast<unsigned short>(l);
-                }
-                if (lane == n) {
-                    run += __popc(hit);
-                    lrun += __popc(hit);
-                }
-            }
-            const int group_images = __shfl_sync(0xffffffffu, incl, 31);
-            if (lane == kBoundaryCounter) run += __popc(any);
-            if (lane == kImageCounter) run += group_images;
-        }
-        if (lane == kStepStay) run += __popc(bs_);
-        if (lane == kStepEmig) run += __popc(be);
-    }
+    const MoveTile t = index_move(G, s, word, base, ghosts, index_outputs, S, O);
     // forces of the stays read from HBM (not staged), in flight with the copies
     double fstay[ITEMS][3];
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
         fstay[j][0] = fstay[j][1] = fstay[j][2] = 0.0;
-        if (DIRECT_FORCES && dest[j] == s) {
-            const long long src = src_off + wbegin + j * 32 + lane;
+        if (DIRECT_FORCES && t.ni[j] >= 0) {
+            const long long src = src_off + begin + (warp * ITEMS + j) * 32 + lane;
             fstay[j][0] = ro(A.d[6] + src);
             fstay[j][1] = ro(A.d[7] + src);
             fstay[j][2] = ro(A.d[8] + src);
@@ -2404,75 +2382,33 @@ __global__ void __launch_bounds__(NT, 3) k_step_move_staged(
     const int* fseg = s_seg + 13;
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-        if (dest[j] != s) continue;
-        const int l = wbegin + j * 32 + lane - begin;
+        if (t.ni[j] < 0) continue;
+        const int l = (warp * ITEMS + j) * 32 + lane;
         if (FULL && DIRECT_FORCES) {
-            move_from_stage_forces(G, A, s_rec, sg, fseg, l, dst_off + nis[j], fstay[j][0],
+            move_from_stage_forces(G, A, s_rec, sg, fseg, l, dst_off + t.ni[j], fstay[j][0],
                                    fstay[j][1], fstay[j][2]);
         } else if (FULL) {
-            move_from_stage(G, A, s_rec, sg, fseg, l, dst_off + nis[j]);
+            move_from_stage(G, A, s_rec, sg, fseg, l, dst_off + t.ni[j]);
         } else {
             for (int c = a0; c < a1; ++c)
-                move_array_from_stage(G, A, s_rec, s_seg[c - a0], c, l, dst_off + nis[j]);
+                move_array_from_stage(G, A, s_rec, s_seg[c - a0], c, l, dst_off + t.ni[j]);
         }
     }
     if (!ghosts) return;
     const double* shift = G.shift + static_cast<long long>(s) * kMaxNeighbors * 3;
-    if (staged) {
-        // list by list: consecutive threads write consecutive ghost slots
-        for (int q = threadIdx.x; q < Q; q += NT) {
-            int lo = 0, hi = nn;
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (s_off[mid] <= q) lo = mid;
-                else hi = mid;
-            }
-            const int n = lo;
-            const int slot = s_base[n] + (q - s_off[n]);
-            const int l = s_own[q];
-            if (FULL) {
-                ghost_from_stage(G, A, s_rec, sg, fseg, l, ghost_off + slot, shift + 3 * n);
-            } else {
-                for (int c = a0; c < a1; ++c)
-                    ghost_array_from_stage(G, A, s_rec, s_seg[c - a0], c, l, ghost_off + slot,
-                                           shift + 3 * n);
-            }
-            if (index_outputs) {
-                ghost_owner[slot] = s_ni[l];
-                ghost_entry[slot] = s * kMaxNeighbors + n;
-            }
+    each_image(t, S, [&](int n, int slot, int l) {
+        if (FULL) {
+            ghost_from_stage(G, A, s_rec, sg, fseg, l, ghost_off + slot, shift + 3 * n);
+        } else {
+            for (int c = a0; c < a1; ++c)
+                ghost_array_from_stage(G, A, s_rec, s_seg[c - a0], c, l, ghost_off + slot,
+                                       shift + 3 * n);
         }
-        return;
-    }
-    // a tile with more images than the staging holds (a halo wider than
-    // half a cell) writes them from the hitting lanes directly
-    run = run0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int l = wbegin + j * 32 + lane - begin;
-        const unsigned mj = msk[j];
-        const unsigned used = __reduce_or_sync(0xffffffffu, mj);
-        for (unsigned rest = used; rest; rest &= rest - 1) {
-            const int n = __ffs(rest) - 1;
-            const unsigned hit = __ballot_sync(0xffffffffu, (mj >> n) & 1u);
-            const int list_base = __shfl_sync(0xffffffffu, run, n);
-            if ((mj >> n) & 1u) {
-                const int slot = list_base + __popc(hit & lt);
-                if (FULL) {
-                    ghost_from_stage(G, A, s_rec, sg, fseg, l, ghost_off + slot, shift + 3 * n);
-                } else {
-                    for (int c = a0; c < a1; ++c)
-                        ghost_array_from_stage(G, A, s_rec, s_seg[c - a0], c, l, ghost_off + slot,
-                                               shift + 3 * n);
-                }
-                if (index_outputs) {
-                    ghost_owner[slot] = nis[j];
-                    ghost_entry[slot] = s * kMaxNeighbors + n;
-                }
-            }
-            if (lane == n) run += __popc(hit);
+        if (index_outputs) {
+            O.ghost_owner[slot] = S.ni[l];
+            O.ghost_entry[slot] = s * kMaxNeighbors + n;
         }
-    }
+    });
 }
 
 // ------------------------------------------------------- walks of the ghosts
@@ -3631,17 +3567,17 @@ void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, con
     case 64:
         pdl_launch(pick(k_step_classify<64, 16, false>, k_step_classify<64, 16, true>), G.max_tiles, 64, 0, s,
             G, x, y, z, S.cnt, S.stride, S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.dest16,
-            S.mask, S.pairs);
+            S.bits, S.pairs);
         break;
     case 256:
         pdl_launch(pick(k_step_classify<256, 5, false>, k_step_classify<256, 5, true>), G.max_tiles, 256, 0, s,
             G, x, y, z, S.cnt, S.stride, S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.dest16,
-            S.mask, S.pairs);
+            S.bits, S.pairs);
         break;
     default:
         pdl_launch(pick(k_step_classify<128, 12, false>, k_step_classify<128, 12, true>), G.max_tiles, 128, 0, s,
             G, x, y, z, S.cnt, S.stride, S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.dest16,
-            S.mask, S.pairs);
+            S.bits, S.pairs);
     }
 }
 
@@ -3651,8 +3587,8 @@ void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s) {
                  S.halo_info, S.cbase, S.cbase_imm, S.imm_tile_start, S.imm_tiles};
     pdl_launch(k_step_scan_layout, kStepCounters, 1024, 0, s, G, S.cnt, S.pre, S.stride, T, S.ticket);
     pdl_launch(k_tile_bases, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
-        G, S.pre, S.stride, S.cbase, S.tile_bases, S.imm_total, S.imm_base, S.imm_tile_start,
-        S.imm_tiles);
+        G, S.pre, S.stride, S.cbase, S.tile_bases, S.bits, S.dest16, S.emig_src, S.emig_dst,
+        S.imm_total, S.imm_base, S.imm_tile_start, S.imm_tiles);
 }
 
 int staged_move_modes(const Arrays& A) {
@@ -3682,38 +3618,23 @@ void launch_step_move(const Grid& G, const Arrays& A, long long src_off, long lo
     const int whole = staged_bytes(A);
     int ends[kStagedArrays], passes = 0;
     const bool split = staged_passes(A, ends, passes);
-    auto staged = [&](bool full, int a0, int a1, int index_outputs) {
-        const int bytes = staged_range_bytes(A, a0, a1);
-        if (full)
-            pdl_launch(k_step_move_staged<true, false>, G.max_tiles, NT, bytes, s,
-                G, A, src_off, dst_off, ghost_off, S.pre, S.stride, S.cbase, S.dest16, S.mask,
-                S.tile_bases, S.emig_src, S.emig_dst, S.ghost_owner, S.ghost_entry, S.bowner,
-                S.boff, S.bslot, S.bfirst, a0, a1, index_outputs);
-        else
-            pdl_launch(k_step_move_staged<false, false>, G.max_tiles, NT, bytes, s,
-                G, A, src_off, dst_off, ghost_off, S.pre, S.stride, S.cbase, S.dest16, S.mask,
-                S.tile_bases, S.emig_src, S.emig_dst, S.ghost_owner, S.ghost_entry, S.bowner,
-                S.boff, S.bslot, S.bfirst, a0, a1, index_outputs);
+    const MoveOutputs O{S.ghost_owner, S.ghost_entry, S.bowner, S.boff, S.bslot, S.bfirst};
+    auto staged = [&](auto kernel, int bytes, int a0, int a1, int index_outputs) {
+        pdl_launch(kernel, G.max_tiles, NT, bytes, s, G, A, src_off, dst_off, ghost_off, S.bits,
+                   S.tile_bases, O, a0, a1, index_outputs);
     };
     if (S.move_staged == 3 && whole - kForceStageBytes <= kStagedMaxBytes) {
-        pdl_launch(k_step_move_staged<true, true>, G.max_tiles, NT, whole - kForceStageBytes, s,
-            G, A, src_off, dst_off, ghost_off, S.pre, S.stride, S.cbase, S.dest16, S.mask,
-            S.tile_bases, S.emig_src, S.emig_dst, S.ghost_owner, S.ghost_entry, S.bowner, S.boff,
-            S.bslot, S.bfirst, 0, narrays, 1);
-    } else if (S.move_staged == 1 && whole <= kStagedMaxBytes) {
-        staged(true, 0, narrays, 1);
+        staged(k_step_move_staged<true, true>, whole - kForceStageBytes, 0, narrays, 1);
+    } else if ((S.move_staged == 1 && whole <= kStagedMaxBytes) ||
+               (S.move_staged != 0 && split && passes == 1)) {
+        staged(k_step_move_staged<true, false>, whole, 0, narrays, 1);
     } else if (S.move_staged != 0 && split) {
-        if (passes == 1) {
-            staged(true, 0, narrays, 1);
-        } else {
-            for (int p = 0, a0 = 0; p < passes; a0 = ends[p++])
-                staged(false, a0, ends[p], p == 0 ? 1 : 0);
-        }
+        for (int p = 0, a0 = 0; p < passes; a0 = ends[p++])
+            staged(k_step_move_staged<false, false>, staged_range_bytes(A, a0, ends[p]), a0, ends[p],
+                   p == 0 ? 1 : 0);
     } else {
-        pdl_launch(k_step_move, G.max_tiles, NT, 0, s, G, A, src_off, dst_off, ghost_off, S.pre, S.stride,
-                                               S.cbase, S.dest16, S.mask, S.emig_src, S.emig_dst,
-                                               S.ghost_owner, S.ghost_entry, S.bowner, S.boff,
-                                               S.bslot, S.bfirst);
+        pdl_launch(k_step_move, G.max_tiles, NT, 0, s, G, A, src_off, dst_off, ghost_off, S.bits,
+                   S.tile_bases, O);
     }
 }
 
@@ -3739,8 +3660,8 @@ void launch_step_export(const Grid& G, const Scratch& S, int* out, cudaStream_t 
 
 void launch_step_bases(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s) {
     pdl_launch(k_tile_bases, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
-        G, S.pre, S.stride, S.cbase, S.tile_bases, imm_in, S.imm_base, S.imm_tile_start,
-        S.imm_tiles);
+        G, S.pre, S.stride, S.cbase, S.tile_bases, S.bits, S.dest16, S.emig_src, S.emig_dst, imm_in,
+        S.imm_base, S.imm_tile_start, S.imm_tiles);
 }
 
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,

@@ -40,7 +40,8 @@ struct Scratch {
     int* emig_info = nullptr;  // {E, nchunks}
     long long* mig_results = nullptr;  // [P][6]
     unsigned* mask = nullptr;  // [ncap] halo neighbor mask per owned particle
-    unsigned short* dest16 = nullptr;  // [max_tiles * 512] destination per tile slot (fused step)
+    unsigned* bits = nullptr;          // [max_tiles * 128] halo, stay and leave bits (fused step)
+    unsigned short* dest16 = nullptr;  // [max_tiles * 512] destination of the leavers, per tile slot
     int* tile_bases = nullptr;         // [max_tiles * 32] step counter bases per tile
     int* out_flags = nullptr;          // [P] out-of-domain flags
     int* list_len = nullptr;   // [P*26] send-list lengths
