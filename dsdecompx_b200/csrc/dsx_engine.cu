@@ -474,6 +474,11 @@ struct dsx_grid {
     // callback does not wait for it (fork and join events, side stream)
     cudaStream_t side_stream = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+    // the emigrants' and immigrants' kernels beside the step's move, on a
+    // stream of the highest priority: their few blocks go in as the move's
+    // many retire, instead of after all of them
+    cudaStream_t emigrant_stream = nullptr;
+    cudaEvent_t emigrant_fork = nullptr, emigrant_join = nullptr;
     bool async_inflight = false;                  // a step whose status is unchecked
     int async_parity = 0;
     unsigned async_status = 0;                    // bits of the checked asynchronous steps
@@ -487,6 +492,9 @@ struct dsx_grid {
         if (fork_ev) cudaEventDestroy(fork_ev);
         if (join_ev) cudaEventDestroy(join_ev);
         if (side_stream) cudaStreamDestroy(side_stream);
+        if (emigrant_fork) cudaEventDestroy(emigrant_fork);
+        if (emigrant_join) cudaEventDestroy(emigrant_join);
+        if (emigrant_stream) cudaStreamDestroy(emigrant_stream);
         if (pinned_build) cudaFreeHost(pinned_build);
         free_shard_buffers();
         for (auto& e : marks.ev) if (e) cudaEventDestroy(e);
@@ -633,6 +641,11 @@ struct dsx_grid {
         cuda_check(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming), "create event");
         cuda_check(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming), "create event");
         cuda_check(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking), "create stream");
+        int lowest = 0, highest = 0;
+        cuda_check(cudaDeviceGetStreamPriorityRange(&lowest, &highest), "stream priorities");
+        cuda_check(cudaStreamCreateWithPriority(&emigrant_stream, cudaStreamNonBlocking, highest), "create stream");
+        cuda_check(cudaEventCreateWithFlags(&emigrant_fork, cudaEventDisableTiming), "create event");
+        cuda_check(cudaEventCreateWithFlags(&emigrant_join, cudaEventDisableTiming), "create event");
         S.marks = &marks;
         last_ghosts.assign(static_cast<std::size_t>(P), 0);
     }
@@ -966,7 +979,9 @@ struct dsx_grid {
             G.need = d_need_empty;
             dsx::launch_step_classify(G, A, owned_off(), S, stream);
             dsx::launch_step_layout(G, S, stream);
+            dsx::launch_step_bases(G, S, stream);
             dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);
+            dsx::launch_step_emigrant_list(G, S, S.imm_total, stream);
             dsx::launch_step_emigrants(G, A, owned_off(), next_off(), S, S.imm_total, nullptr, stream);
         }
         commit_migrate();
@@ -1245,7 +1260,10 @@ struct dsx_grid {
             cur ^= 1;
             const dsx::Grid Gn = params();
             cur ^= 1;
-            dsx::launch_fused_step(G, Gn, A, owned_off(), next_off(), ghost_off(), S, stream, dynamic);
+            // one stream when every kernel is timed by itself
+            const dsx::Branch branch{emigrant_stream, emigrant_fork, emigrant_join};
+            cuda_check(dsx::launch_fused_step(G, Gn, A, owned_off(), next_off(), ghost_off(), S, stream,
+                                              dynamic, marks.on ? nullptr : &branch), "launch step");
         }
         if (build_event) {
             // the build's status and totals, then the event the next
@@ -1272,6 +1290,7 @@ struct dsx_grid {
         plan_valid = saved_plan;
         ghosts_valid = saved_ghosts;
         marks.mark(stream, "callback");
+        if (!marks.on) dsx::plain_edge();   // the callback may have queued nothing after the join
         enqueue_reverse(stream);
         // the status after the build is the step's (nothing later sets a
         // bit): a step with the build's copy needs no second one
@@ -1529,6 +1548,7 @@ struct dsx_grid {
                 clear_status(stream);
                 dsx::launch_step_classify(G, A, src, S, stream);
                 dsx::launch_step_layout(G, S, stream);
+                dsx::launch_step_bases(G, S, stream);
                 const unsigned st = read_status(stream);
                 if (!(st & dsx::kStatusGhostOverflow)) break;
                 grow_ghosts(static_cast<long long>(static_cast<int>(pinned_status[1])), stream);
@@ -1977,7 +1997,8 @@ struct dsx_grid {
         // stays and ghost images of the retained particles, then the
         // emigrants in the reference's order with gaps for other shards'
         const dsx::Grid Gp = params();
-        dsx::launch_step_bases(Gp, S, d_imm_tiles_in, stream);
+        dsx::launch_step_bases(Gp, S, stream);
+        dsx::launch_step_emigrant_list(Gp, S, d_imm_tiles_in, stream);
         dsx::launch_step_move(Gp, A, owned_off(), next_off(), ghost_off(), S, stream);
         dsx::launch_step_emigrants(Gp, A, owned_off(), next_off(), S, d_local_imm, S.gap, stream);
         std::vector<int> all(static_cast<std::size_t>(13 + fields.size()));
@@ -2793,10 +2814,10 @@ int dsx_grid_kernel_times(dsx_grid* grid, int max, const char** names, float* ms
 }
 
 int dsx_grid_step_kernel_count(dsx_grid* grid) {
-    // rebalance (Dynamic only); classify, counter scan, layout, tile bases,
-    // move; emigrant histogram, column scan, placement; immigrants' classify,
-    // scan, scatter; reverse sum
-    return (grid->desc.policy == DSX_DYNAMIC ? 1 : 0) + 5 + 3 + 3 + 1;
+    // rebalance (Dynamic only); classify, counter scan with the layout, tile
+    // bases, move; emigrant list, histogram, column scan, placement;
+    // immigrants' classify, scan, scatter; reverse sum
+    return (grid->desc.policy == DSX_DYNAMIC ? 1 : 0) + 4 + 4 + 3 + 1;
 }
 
 }  // extern "C"

@@ -2252,39 +2252,45 @@ __device__ __forceinline__ void fill_tiles_grid(int P, int tile, const int* n, c
 }
 
 // Counter bases of every tile of the layout (30 per tile, row stride 32), so
-// that the move reads them with one load per tile; the list of emigrants, in
-// (source subdomain, source order); and the tile descriptors of the next
-// layout and of its immigrant segments (imm_in: immigrants per subdomain,
-// imm_base: where they start, imm_ts: their tile starts).  A warp per tile.
+// that the move reads them with one load per tile.
 __global__ void __launch_bounds__(NT) k_tile_bases(Grid G, const int* pre, int stride,
-                                                   const int* cbase_ret, int* tile_bases,
-                                                   const unsigned* __restrict__ bits,
-                                                   const unsigned short* __restrict__ dest,
-                                                   int* emig_src, int* emig_dst,
-                                                   const int* imm_in, const int* imm_base,
-                                                   const int* imm_ts, int4* imm_tiles) {
+                                                   const int* cbase_ret, int* tile_bases) {
+    pdl_begin();
+    const int ntiles = G.tile_start[G.P];
+    for (long long idx = blockIdx.x * static_cast<long long>(NT) + threadIdx.x;
+         idx < static_cast<long long>(ntiles) * 32; idx += static_cast<long long>(gridDim.x) * NT) {
+        const int g = static_cast<int>(idx >> 5), k = static_cast<int>(idx & 31);
+        if (k < kStepCounters) tile_bases[idx] = tile_base(G, pre, stride, cbase_ret, g, G.tiles[g], k);
+    }
+}
+
+// The list of emigrants, in (source subdomain, source order), from the tiles'
+// leave bits and the scanned counter (a warp per tile); and the tile
+// descriptors of the next layout and of its immigrant segments (imm_in:
+// immigrants per subdomain, imm_base: where they start, imm_ts: their tile
+// starts).  Nothing here waits for the move, so the emigrants' chain of
+// kernels runs beside it.
+__global__ void __launch_bounds__(NT) k_emig_list(Grid G, const int* pre, int stride,
+                                                  const unsigned* __restrict__ bits,
+                                                  const unsigned short* __restrict__ dest,
+                                                  int* emig_src, int* emig_dst, const int* imm_in,
+                                                  const int* imm_base, const int* imm_ts,
+                                                  int4* imm_tiles) {
     pdl_begin();
     const int ntiles = G.tile_start[G.P];
     const int lane = threadIdx.x & 31;
     for (int g = blockIdx.x * NW + (threadIdx.x >> 5); g < ntiles; g += gridDim.x * NW) {
-        const int4 td = G.tiles[g];
-        const long long slot0 = static_cast<long long>(g) * TILE + lane * 32;
+        const int begin = G.tiles[g].y;
+        const int first = pre[kStepEmig * stride + g];
         unsigned leave = lane < kGroups
             ? ro(bits + static_cast<long long>(g) * kTileWords + lane * kGroupWords + kLeaveWord) : 0u;
-        int first = 0;
-        if (lane < kStepCounters) {
-            first = tile_base(G, pre, stride, cbase_ret, g, td, lane);
-            tile_bases[static_cast<long long>(g) * 32 + lane] = first;
-        }
-        const int emigrants = __shfl_sync(0xffffffffu, first, kStepEmig);
-        if (__any_sync(0xffffffffu, leave != 0)) {
-            const int c = __popc(leave);
-            int e = emigrants + warp_inclusive_sum(c) - c;
-            for (; leave; leave &= leave - 1, ++e) {
-                const int l = __ffs(leave) - 1;
-                emig_src[e] = td.y + lane * 32 + l;
-                emig_dst[e] = dest[slot0 + l];
-            }
+        if (!__any_sync(0xffffffffu, leave != 0)) continue;
+        const int c = __popc(leave);
+        int e = first + warp_inclusive_sum(c) - c;
+        for (; leave; leave &= leave - 1, ++e) {
+            const int l = lane * 32 + __ffs(leave) - 1;
+            emig_src[e] = begin + l;
+            emig_dst[e] = dest[static_cast<long long>(g) * TILE + l];
         }
     }
     fill_tiles_grid(G.P, G.tile, G.n_next, G.obase_next, G.tile_start_next, G.tiles_next);
@@ -3383,6 +3389,13 @@ int sm_count() {
 // the kernel's CTAs become resident (and then wait, pdl_begin) while the
 // previous kernel on the stream drains, inside captured graphs too; errors
 // surface through cudaGetLastError like those of triple-chevron launches.
+//
+// The first kernel on a stream after it was joined with another one waits for
+// both in full: a PlainEdge in scope makes the next launch of this thread an
+// ordinary one (the attribute orders a kernel against its stream's own
+// predecessor only).
+thread_local bool t_plain_edge = false;
+
 template <class... Params, class... Args>
 void pdl_launch(void (*kernel)(Params...), dim3 grid, int block, std::size_t smem, cudaStream_t s,
                 Args&&... args) {
@@ -3395,7 +3408,8 @@ void pdl_launch(void (*kernel)(Params...), dim3 grid, int block, std::size_t sme
     config.dynamicSmemBytes = smem;
     config.stream = s;
     config.attrs = attr;
-    config.numAttrs = 1;
+    config.numAttrs = t_plain_edge ? 0 : 1;
+    t_plain_edge = false;
     (void)cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
@@ -3586,9 +3600,17 @@ void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s) {
                  S.mig_results, S.list_ret, S.list_len, S.send_base, S.list_flat, S.g, S.gbase, S.boff,
                  S.halo_info, S.cbase, S.cbase_imm, S.imm_tile_start, S.imm_tiles};
     pdl_launch(k_step_scan_layout, kStepCounters, 1024, 0, s, G, S.cnt, S.pre, S.stride, T, S.ticket);
+}
+
+void launch_step_bases(const Grid& G, const Scratch& S, cudaStream_t s) {
     pdl_launch(k_tile_bases, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
-        G, S.pre, S.stride, S.cbase, S.tile_bases, S.bits, S.dest16, S.emig_src, S.emig_dst,
-        S.imm_total, S.imm_base, S.imm_tile_start, S.imm_tiles);
+        G, S.pre, S.stride, S.cbase, S.tile_bases);
+}
+
+void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s) {
+    pdl_launch(k_emig_list, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
+        G, S.pre, S.stride, S.bits, S.dest16, S.emig_src, S.emig_dst, imm_in, S.imm_base,
+        S.imm_tile_start, S.imm_tiles);
 }
 
 int staged_move_modes(const Arrays& A) {
@@ -3658,14 +3680,9 @@ void launch_step_export(const Grid& G, const Scratch& S, int* out, cudaStream_t 
     pdl_launch(k_step_export, 1, 1024, 0, s, G, S.pre, S.stride, out);
 }
 
-void launch_step_bases(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s) {
-    pdl_launch(k_tile_bases, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
-        G, S.pre, S.stride, S.cbase, S.tile_bases, S.bits, S.dest16, S.emig_src, S.emig_dst, imm_in,
-        S.imm_base, S.imm_tile_start, S.imm_tiles);
-}
-
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
                         long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s) {
+    launch_step_emigrant_list(G, S, S.imm_total, s);
     launch_step_emigrants(G, A, src_off, dst_off, S, S.imm_total, nullptr, s);
     launch_step_immigrant_halo(Gn, A, dst_off, ghost_off, S, s);
 }
@@ -3686,17 +3703,44 @@ void launch_step_immigrant_halo(const Grid& Gn, const Arrays& A, long long dst_o
                                            S.boff, S.bslot, S.bfirst);
 }
 
-void launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
-                       long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s,
-                       bool counters_zeroed) {
+cudaError_t fork_branch(const Branch& b, cudaStream_t s) {
+    cudaError_t e = cudaEventRecord(b.fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(b.stream, b.fork, 0);
+    t_plain_edge = true;
+    return e;
+}
+
+cudaError_t join_branch(const Branch& b, cudaStream_t s) {
+    cudaError_t e = cudaEventRecord(b.join, b.stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b.join, 0);
+    return e;
+}
+
+void plain_edge() { t_plain_edge = true; }
+
+cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
+                              long long dst_off, long long ghost_off, const Scratch& S,
+                              cudaStream_t s, bool counters_zeroed, const Branch* branch) {
     launch_step_classify(G, A, src_off, S, s, counters_zeroed);
     if (S.marks) S.marks->mark(s, "step_classify");
     launch_step_layout(G, S, s);
+    if (branch) {
+        // the emigrants' and the immigrants' kernels read what the layout
+        // left and write slots the move does not: they run beside it
+        cudaError_t e = fork_branch(*branch, s);
+        launch_step_finish(G, Gn, A, src_off, dst_off, ghost_off, S, branch->stream);
+        launch_step_bases(G, S, s);
+        launch_step_move(G, A, src_off, dst_off, ghost_off, S, s);
+        const cudaError_t j = join_branch(*branch, s);
+        return e != cudaSuccess ? e : j;
+    }
+    launch_step_bases(G, S, s);
     if (S.marks) S.marks->mark(s, "step_layout");
     launch_step_move(G, A, src_off, dst_off, ghost_off, S, s);
     if (S.marks) S.marks->mark(s, "step_move");
     launch_step_finish(G, Gn, A, src_off, dst_off, ghost_off, S, s);
     if (S.marks) S.marks->mark(s, "immigrant_halo");
+    return cudaSuccess;
 }
 
 // Shared memory of one tile of the arrays a refresh copies (x, y, z; with

@@ -107,19 +107,38 @@ void launch_halo_build(const Grid& G, const Arrays& A, long long owned_off,
                        long long ghost_off, const Scratch& S, cudaStream_t s,
                        const PlainLaunch* plain = nullptr);
 
+// A second stream for kernels that run beside others: fork makes it follow
+// what `s` holds so far, join makes `s` follow it.  The next launch of the
+// calling thread after a fork is ordinary (no programmatic edge); plain_edge()
+// asks the same for the first launch on a joined stream.
+struct Branch {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+cudaError_t fork_branch(const Branch& b, cudaStream_t s);
+cudaError_t join_branch(const Branch& b, cudaStream_t s);
+void plain_edge();
+
 // migrate + plan build as one pipeline (the batched step); G: current layout,
-// Gn: the same grid with the next layout current.
-void launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
-                       long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s,
-                       bool counters_zeroed = false);
+// Gn: the same grid with the next layout current.  branch: where the
+// emigrants' and immigrants' kernels run beside the move (joined on return),
+// or null for one stream.
+cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
+                              long long dst_off, long long ghost_off, const Scratch& S,
+                              cudaStream_t s, bool counters_zeroed = false,
+                              const Branch* branch = nullptr);
 
 // The pipeline's parts, in order (the autotuner replays them one by one):
 // classify (destinations, masks, tile counters), the counter scan and the
-// next layout, the move (idempotent for a fixed current half), and the
-// emigrant placement plus the immigrants' ghost images.
+// next layout, the tiles' counter bases, the move (idempotent for a fixed
+// current half), and the emigrants' list and placement plus the immigrants'
+// ghost images.
 void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, const Scratch& S,
                           cudaStream_t s, bool counters_zeroed = false);
 void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s);
+void launch_step_bases(const Grid& G, const Scratch& S, cudaStream_t s);
+// imm_in: immigrants per subdomain whose ghost images this grid makes
+void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s);
 void launch_step_move(const Grid& G, const Arrays& A, long long src_off, long long dst_off,
                       long long ghost_off, const Scratch& S, cudaStream_t s);
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
@@ -133,12 +152,10 @@ void launch_step_emigrants(const Grid& G, const Arrays& A, long long src_off, lo
 void launch_step_immigrant_halo(const Grid& Gn, const Arrays& A, long long dst_off,
                                 long long ghost_off, const Scratch& S, cudaStream_t s);
 // A sharded step's pieces around its host-planned layout: the counter scan
-// alone, the per-subdomain export of the scanned counters (29 P + 1 ints, see
-// k_step_export), and the tile bases and descriptors of the planned layout
-// (imm_in: immigrants per subdomain whose ghost images this grid makes).
+// alone, and the per-subdomain export of the scanned counters (29 P + 1 ints,
+// see k_step_export).
 void launch_step_scan(const Grid& G, const Scratch& S, cudaStream_t s);
 void launch_step_export(const Grid& G, const Scratch& S, int* out, cudaStream_t s);
-void launch_step_bases(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s);
 // Move kinds that apply to this record, as bits: 1 direct reads (kind 0),
 // 2 staged (kind 1: one pass when a tile of the record fits 100 KB of shared
 // memory, else passes of at most 56 KB), 4 staged in passes although one
