@@ -773,6 +773,10 @@ struct dsx_grid {
         S.imm_list = S.imm_total + P;
         S.imm_bnd = S.imm_list + static_cast<std::size_t>(P) * dsx::kMaxNeighbors;
         S.imm_img = S.imm_bnd + P;
+        S.imm_copies = dsx::immigrant_copies(P);
+        const std::size_t nrep = static_cast<std::size_t>(P) * (3 + dsx::kMaxNeighbors) * S.imm_copies;
+        S.imm_rep = device_alloc<int>(fixed_owned, nrep);
+        cuda_check(cudaMemset(S.imm_rep, 0, nrep * sizeof(int)), "memset");
         S.list_ret = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * E);
         S.cbase_imm = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * dsx::kHaloCounters);
         S.imm_tile_start = device_alloc<int>(fixed_owned, P + 1);
@@ -885,8 +889,8 @@ struct dsx_grid {
         plain_bounds[static_cast<std::size_t>(P)] = info[1];
     }
 
-    // first_of_step: the batched step's rebalance, which also clears the
-    // status word and the step's immigrant counters (their memsets skipped)
+    // first_of_step: the rebalance that opens a step or a migrate, which also
+    // clears the status word (on other grids the layout stores it)
     void enqueue_rebalance(cudaStream_t stream, bool automatic_rebalance,
                            const double* work_in = nullptr, bool first_of_step = false) {
         const dsx::Grid G = params();
@@ -901,11 +905,7 @@ struct dsx_grid {
             p.halo_width = halo_width;
             p.automatic = 1;
             p.interval = automatic_rebalance ? static_cast<long long>(desc.dyn_interval) : 0;
-            if (first_of_step) {
-                p.clear_status = 1;
-                p.zero = S.imm_total;
-                p.nzero = P * (3 + dsx::kMaxNeighbors);
-            }
+            p.clear_status = first_of_step ? 1 : 0;
             dsx::launch_rebalance(G, work_in, p, call_counter, rebalance_result, stream);
             dsx::mark(S, stream, "rebalance");
         }
@@ -953,7 +953,6 @@ struct dsx_grid {
 
     void migrate(cudaStream_t stream, long long* results, bool automatic_rebalance = true) {
         not_pending("migrate");
-        clear_status(stream);
         // work supplied for this migrate's automatic rebalance (pageable
         // source: the copy is staged before the call returns)
         const double* work_in = nullptr;
@@ -965,11 +964,12 @@ struct dsx_grid {
         }
         if (plain) {
             // the rebalance may move the cut planes but not the layout
+            clear_status(stream);
             enqueue_rebalance(stream, automatic_rebalance, work_in);
             dsx::launch_migrate(params(), A, owned_off(), next_off(), S, stream,
                                 plain_layout(stream));
         } else {
-            enqueue_rebalance(stream, automatic_rebalance, work_in);
+            enqueue_rebalance(stream, automatic_rebalance, work_in, true);
             // the batched step's classify, layout and staged move over an
             // empty halo table: every halo mask is 0, so the pipeline lays
             // out and writes no ghost and leaves what migrate alone leaves
@@ -978,7 +978,7 @@ struct dsx_grid {
             G.lut = d_lut_empty;
             G.need = d_need_empty;
             dsx::launch_step_classify(G, A, owned_off(), S, stream);
-            dsx::launch_step_layout(G, S, stream);
+            dsx::launch_step_layout(G, S, stream, desc.policy != DSX_DYNAMIC);
             dsx::launch_step_bases(G, S, stream);
             dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);
             dsx::launch_step_emigrant_list(G, S, S.imm_total, stream);
@@ -1249,10 +1249,9 @@ struct dsx_grid {
 
     void enqueue_step(dsx_step_callback cb, void* user, cudaStream_t stream, bool build_event = false) {
         marks.count = 0;
-        // a Dynamic grid's rebalance opens the step and clears the status and
-        // the immigrant counters itself
+        // a Dynamic grid's rebalance opens the step and clears the status;
+        // elsewhere the layout is the first to set it, and stores it
         const bool dynamic = desc.policy == DSX_DYNAMIC;
-        if (!dynamic) clear_status(stream);
         marks.mark(stream, "start");
         enqueue_rebalance(stream, true, nullptr, dynamic);
         {
@@ -1263,7 +1262,7 @@ struct dsx_grid {
             // one stream when every kernel is timed by itself
             const dsx::Branch branch{emigrant_stream, emigrant_fork, emigrant_join};
             cuda_check(dsx::launch_fused_step(G, Gn, A, owned_off(), next_off(), ghost_off(), S, stream,
-                                              dynamic, marks.on ? nullptr : &branch), "launch step");
+                                              !dynamic, marks.on ? nullptr : &branch), "launch step");
         }
         if (build_event) {
             // the build's status and totals, then the event the next
@@ -1533,7 +1532,7 @@ struct dsx_grid {
                 for (int i = 0; i < 3; ++i) {
                     S.classify_threads = shapes[i];
                     S.classify_combine = c;
-                    const float ms = time([&] { dsx::launch_step_classify(G, A, src, S, stream); });
+                    const float ms = time([&] { dsx::launch_step_classify(G, A, src, S, stream, true); });
                     (c ? r.classify_combined_ms : r.classify_ms)[i] = ms;
                     if (best_classify < 0.0f || ms < best_classify) {
                         best_classify = ms;
@@ -1546,7 +1545,7 @@ struct dsx_grid {
             // the next layout's plan; the ghost region grows until it fits
             for (;;) {
                 clear_status(stream);
-                dsx::launch_step_classify(G, A, src, S, stream);
+                dsx::launch_step_classify(G, A, src, S, stream, true);
                 dsx::launch_step_layout(G, S, stream);
                 dsx::launch_step_bases(G, S, stream);
                 const unsigned st = read_status(stream);
@@ -1617,7 +1616,7 @@ struct dsx_grid {
                 cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
                 enqueue_step(cb, user, stream, true);
                 cuda_check(cudaStreamEndCapture(stream, &g), "end capture");
-                cuda_check(cudaGraphInstantiate(&exec, g, 0), "instantiate graph");
+                cuda_check(cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority), "instantiate graph");
                 cudaGraphDestroy(g);
             }
             cuda_check(cudaGraphLaunch(exec, stream), "launch graph");
@@ -1676,7 +1675,7 @@ struct dsx_grid {
             cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
             enqueue_step(cb, user, stream, true);
             cuda_check(cudaStreamEndCapture(stream, &g), "end capture");
-            cuda_check(cudaGraphInstantiate(&exec, g, 0), "instantiate graph");
+            cuda_check(cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority), "instantiate graph");
             cudaGraphDestroy(g);
         }
         const int p = parity;

@@ -1068,24 +1068,59 @@ __device__ __forceinline__ unsigned halo_flags(const TileBounds& b, double px, d
            (py > b.hi[1] ? 8u : 0u) | (pz < b.lo[2] ? 16u : 0u) | (pz > b.hi[2] ? 32u : 0u);
 }
 
+// The immigrant counters of a step, one block of 29 P: per destination the
+// immigrants, their part of each of its send lists, boundary owners, images.
+// The classify adds to `copies` of the block, a tile to copy tile % copies:
+// the leavers of a grid of few subdomains all add to the same few counters,
+// and atomics on one address run one after the other (8M particles in 2x2x2,
+// 96,000 leavers: 160 us with one copy, 57 with 32).  The next kernel
+// (the layout, or a sharded step's export) sums the copies into the block and
+// leaves them zero for the next step.
+constexpr int kImmCounters = 3 + kMaxNeighbors;
+
+struct ImmCounters {
+    int *total, *list, *bnd, *img;
+    __device__ __forceinline__ ImmCounters(int P, int* block)
+        : total(block), list(block + P), bnd(block + (1 + kMaxNeighbors) * P),
+          img(block + (2 + kMaxNeighbors) * P) {}
+};
+
+__device__ __forceinline__ void sum_immigrants(int P, int* imm, int* imm_rep, int copies) {
+    const int n = kImmCounters * P;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        int sum = 0;
+#pragma unroll 8
+        for (int c = 0; c < copies; ++c) {
+            int* at = imm_rep + static_cast<long long>(c) * n + k;
+            sum += __ldcg(at);
+            *at = 0;
+        }
+        imm[k] = sum;
+    }
+    __syncthreads();
+}
+
 // F1: the bits of every owned particle (of the halo of its NEW owner where it
 // stays), destinations of those that leave, per-tile counters, and
 // per-destination totals of the leavers (atomics: only sums; COMBINE: one per
 // destination and warp, add_immigrants).
 //
-// Bound by reading the positions (24 B per particle): with the bits and the
-// lane-parallel counting a group of 32 costs about 70 warp instructions
-// against 220 with a mask and a destination per particle.
+// Bound by reading the positions (24 B per particle) and by what the leavers
+// cost: with the bits and the lane-parallel counting a group of 32 costs about
+// 70 warp instructions against 220 with a mask and a destination per particle
+// (16M clustered particles 110 -> 88 us, 8M in 2x2x2 69 -> 57 us, 27.2M in
+// 8x8x4 174 -> 129 us).
 template <int CT, int MINB, bool COMBINE>
 __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double* __restrict__ x,
                                                       const double* __restrict__ y,
                                                       const double* __restrict__ z, int* cnt,
-                                                      int stride, int* imm_total, int* imm_list,
-                                                      int* imm_bnd, int* imm_img,
+                                                      int stride, int* imm_rep, int copies,
                                                       unsigned short* __restrict__ dest_out,
                                                       unsigned* __restrict__ bits_out,
                                                       int* pairs) {
     pdl_begin();
+    // this tile's copy of the immigrant counters
+    const ImmCounters imm(G.P, imm_rep + static_cast<long long>(blockIdx.x % copies) * kImmCounters * G.P);
     constexpr int CI = TILE / CT;   // 32-particle groups per warp
     constexpr int CW = CT / 32;
     static_assert(CI * CT == TILE && CW >= 1, "tile split");
@@ -1176,18 +1211,18 @@ __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double
                 // emigrants per (destination, source), for a sharded step
                 if (pairs) atomicAdd(&pairs[d * G.P + s], 1);
                 if constexpr (!COMBINE) {
-                    atomicAdd(&imm_total[d], 1);
+                    atomicAdd(&imm.total[d], 1);
                     if (me) {
-                        atomicAdd(&imm_bnd[d], 1);
-                        atomicAdd(&imm_img[d], __popc(me));
+                        atomicAdd(&imm.bnd[d], 1);
+                        atomicAdd(&imm.img[d], __popc(me));
                         for (unsigned r = me; r; r &= r - 1)
-                            atomicAdd(&imm_list[d * kMaxNeighbors + __ffs(r) - 1], 1);
+                            atomicAdd(&imm.list[d * kMaxNeighbors + __ffs(r) - 1], 1);
                     }
                 }
             }
         }
         if constexpr (COMBINE)
-            add_immigrants(d >= 0 && d != s ? d : -1, me, lane, imm_total, imm_bnd, imm_img, imm_list);
+            add_immigrants(d >= 0 && d != s ? d : -1, me, lane, imm.total, imm.bnd, imm.img, imm.list);
     }
     if (nq) __syncthreads();   // uniform: the general path changed the words
     // counters: lane n of a warp its list over the warp's groups
@@ -1242,6 +1277,9 @@ struct StepTables {
     int* cbase_imm;
     int* imm_tile_start;
     int4* imm_tiles;
+    int* imm_rep;
+    int copies;
+    int fresh_status;   // the step's first word of status: stored, not or-ed
 };
 
 __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, int stride,
@@ -1284,6 +1322,8 @@ __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, 
     auto tile_sum = [&](int k, int r) {
         return __ldcg(pre + k * stride + ts_old[r + 1]) - __ldcg(pre + k * stride + ts_old[r]);
     };
+    sum_immigrants(P, T.imm_total, T.imm_rep, T.copies);
+    unsigned status = 0;
     // new owned layout and migration results
     int retained = 0, received = 0, old = 0, next = 0;
     if (t < P) {
@@ -1319,7 +1359,7 @@ __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, 
         const int E = __ldcg(pre + kStepEmig * stride + ntiles);
         T.emig_info[0] = E;
         T.emig_info[1] = (E + TILE - 1) / TILE;
-        if (total_next != G.obase[P]) atomicOr(G.status, kStatusMigrationMismatch);
+        if (total_next != G.obase[P]) status |= kStatusMigrationMismatch;
     }
     // send-list lengths: retained part from the tile prefixes, immigrant part
     // from the atomics of F1
@@ -1402,8 +1442,10 @@ __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, 
         T.gbase[P] = total_ghosts;
         T.info[0] = total_ghosts;
         T.info[1] = total_b;
-        if (static_cast<long long>(total_ghosts) > G.gcap) atomicOr(G.status, kStatusGhostOverflow);
+        if (static_cast<long long>(total_ghosts) > G.gcap) status |= kStatusGhostOverflow;
         else T.boff[total_b] = total_i;
+        if (T.fresh_status) *G.status = status;
+        else if (status) atomicOr(G.status, status);
     }
 }
 
@@ -2302,9 +2344,11 @@ __global__ void __launch_bounds__(NT) k_emig_list(Grid G, const int* pre, int st
 // shard: out[0, P) retained particles, [P, 2P) boundary owners and [2P, 3P)
 // their images (the retained parts), [3P, 3P + 26P) the retained part of
 // every send list, and out[29P] the emigrants of this shard.
-__global__ void __launch_bounds__(1024) k_step_export(Grid G, const int* pre, int stride, int* out) {
+__global__ void __launch_bounds__(1024) k_step_export(Grid G, const int* pre, int stride, int* out,
+                                                      int* imm, int* imm_rep, int copies) {
     pdl_begin();
     const int P = G.P;
+    sum_immigrants(P, imm, imm_rep, copies);
     const int* ts = G.tile_start;
     auto tile_sum = [&](int k, int r) {
         return pre[k * stride + ts[r + 1]] - pre[k * stride + ts[r]];
@@ -2325,6 +2369,11 @@ __global__ void __launch_bounds__(1024) k_step_export(Grid G, const int* pre, in
 // F4 with the tile's records staged in shared memory (same output as
 // k_step_move).  Dynamic shared memory: sum over the arrays of TILE x element
 // bytes + 32.
+//
+// With the index phase on the tile's bits (6 -> 1 B per particle read, and the
+// lists ranked lane-parallel) 27.2M particles of 148 B move in 1.91 ms against
+// 1.98, 16M of 104 B in 0.725 against 0.748, and staging the whole 148 B record
+// beats the stage without forces (1.91 / 2.01 ms).
 //
 // FULL: one pass over the whole record.  Otherwise the pass moves arrays
 // [a0, a1) only (a record too wide for three staged tiles per SM is moved in
@@ -2910,7 +2959,6 @@ __global__ void __launch_bounds__(32) k_rebalance(Grid G, const double* work_in,
     const int lane = threadIdx.x;
     if (blockIdx.x != 0) return;
     if (p.clear_status && lane == 0) *G.status = 0u;
-    for (int k = lane; k < p.nzero; k += 32) p.zero[k] = 0;
     const int P = G.P;
     const int ncuts = G.cut_offset[2] + G.dims[2] + 1;
     // everything the warp reads, in one round trip
@@ -3568,9 +3616,13 @@ bool staged_passes(const Arrays& A, int* ends, int& passes) {
     return true;
 }
 
+int immigrant_copies(int P) { return P >= 256 ? 1 : P >= 8 ? 256 / P : 32; }
+
 void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, const Scratch& S,
-                          cudaStream_t s, bool counters_zeroed) {
-    if (!counters_zeroed) cudaMemsetAsync(S.imm_total, 0, sizeof(int) * G.P * (3 + kMaxNeighbors), s);
+                          cudaStream_t s, bool clear_counters) {
+    // (zero between steps: whoever sums the copies clears them)
+    if (clear_counters)
+        cudaMemsetAsync(S.imm_rep, 0, sizeof(int) * static_cast<std::size_t>(G.P) * kImmCounters * S.imm_copies, s);
     if (S.pairs) cudaMemsetAsync(S.pairs, 0, sizeof(int) * G.P * G.P, s);
     const double* x = A.d[0] + src_off;
     const double* y = A.d[1] + src_off;
@@ -3580,25 +3632,26 @@ void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, con
     switch (S.classify_threads) {
     case 64:
         pdl_launch(pick(k_step_classify<64, 16, false>, k_step_classify<64, 16, true>), G.max_tiles, 64, 0, s,
-            G, x, y, z, S.cnt, S.stride, S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.dest16,
+            G, x, y, z, S.cnt, S.stride, S.imm_rep, S.imm_copies, S.dest16,
             S.bits, S.pairs);
         break;
     case 256:
         pdl_launch(pick(k_step_classify<256, 5, false>, k_step_classify<256, 5, true>), G.max_tiles, 256, 0, s,
-            G, x, y, z, S.cnt, S.stride, S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.dest16,
+            G, x, y, z, S.cnt, S.stride, S.imm_rep, S.imm_copies, S.dest16,
             S.bits, S.pairs);
         break;
     default:
         pdl_launch(pick(k_step_classify<128, 12, false>, k_step_classify<128, 12, true>), G.max_tiles, 128, 0, s,
-            G, x, y, z, S.cnt, S.stride, S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.dest16,
+            G, x, y, z, S.cnt, S.stride, S.imm_rep, S.imm_copies, S.dest16,
             S.bits, S.pairs);
     }
 }
 
-void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s) {
+void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s, bool fresh_status) {
     StepTables T{S.imm_total, S.imm_list, S.imm_bnd, S.imm_img, S.imm_base, S.emig_info,
                  S.mig_results, S.list_ret, S.list_len, S.send_base, S.list_flat, S.g, S.gbase, S.boff,
-                 S.halo_info, S.cbase, S.cbase_imm, S.imm_tile_start, S.imm_tiles};
+                 S.halo_info, S.cbase, S.cbase_imm, S.imm_tile_start, S.imm_tiles, S.imm_rep,
+                 S.imm_copies, fresh_status ? 1 : 0};
     pdl_launch(k_step_scan_layout, kStepCounters, 1024, 0, s, G, S.cnt, S.pre, S.stride, T, S.ticket);
 }
 
@@ -3677,7 +3730,7 @@ void launch_step_scan(const Grid& G, const Scratch& S, cudaStream_t s) {
 }
 
 void launch_step_export(const Grid& G, const Scratch& S, int* out, cudaStream_t s) {
-    pdl_launch(k_step_export, 1, 1024, 0, s, G, S.pre, S.stride, out);
+    pdl_launch(k_step_export, 1, 1024, 0, s, G, S.pre, S.stride, out, S.imm_total, S.imm_rep, S.imm_copies);
 }
 
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
@@ -3720,10 +3773,10 @@ void plain_edge() { t_plain_edge = true; }
 
 cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
                               long long dst_off, long long ghost_off, const Scratch& S,
-                              cudaStream_t s, bool counters_zeroed, const Branch* branch) {
-    launch_step_classify(G, A, src_off, S, s, counters_zeroed);
+                              cudaStream_t s, bool fresh_status, const Branch* branch) {
+    launch_step_classify(G, A, src_off, S, s);
     if (S.marks) S.marks->mark(s, "step_classify");
-    launch_step_layout(G, S, s);
+    launch_step_layout(G, S, s, fresh_status);
     if (branch) {
         // the emigrants' and the immigrants' kernels read what the layout
         // left and write slots the move does not: they run beside it

@@ -33,6 +33,8 @@ struct Scratch {
     int* pre = nullptr;        // [kHaloCounters][stride] exclusive prefixes
     int stride = 0;            // max_tiles + 1
     int* imm_total = nullptr;  // [P] immigrants per destination
+    int* imm_rep = nullptr;    // [imm_copies][29 P] the classify's immigrant counters
+    int imm_copies = 1;
     int* imm_base = nullptr;   // [P]
     int* emig_src = nullptr;   // [ncap]
     int* emig_dst = nullptr;   // [ncap]
@@ -122,10 +124,11 @@ void plain_edge();
 // migrate + plan build as one pipeline (the batched step); G: current layout,
 // Gn: the same grid with the next layout current.  branch: where the
 // emigrants' and immigrants' kernels run beside the move (joined on return),
-// or null for one stream.
+// or null for one stream.  fresh_status: nothing of the step has set a status
+// bit yet, so the layout stores its word (no clearing before it).
 cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
                               long long dst_off, long long ghost_off, const Scratch& S,
-                              cudaStream_t s, bool counters_zeroed = false,
+                              cudaStream_t s, bool fresh_status = false,
                               const Branch* branch = nullptr);
 
 // The pipeline's parts, in order (the autotuner replays them one by one):
@@ -134,8 +137,11 @@ cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, lo
 // current half), and the emigrants' list and placement plus the immigrants'
 // ghost images.
 void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, const Scratch& S,
-                          cudaStream_t s, bool counters_zeroed = false);
-void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s);
+                          cudaStream_t s, bool clear_counters = false);
+void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s, bool fresh_status = false);
+// Copies of the immigrant counters for P subdomains: 256 counters' worth of
+// addresses for each sum where P is small (the layout reads every copy).
+int immigrant_copies(int P);
 void launch_step_bases(const Grid& G, const Scratch& S, cudaStream_t s);
 // imm_in: immigrants per subdomain whose ghost images this grid makes
 void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s);
@@ -202,11 +208,9 @@ struct RebalanceParams {
     int force = 0;
     long long interval = 1;   // 0: automatic rebalance disabled
     int automatic = 0;        // 1: the migrate-time check (counts the call)
-    // the batched step's first kernel also clears the status word and the
-    // step's immigrant counters (instead of two memset nodes before it)
+    // the batched step's first kernel also clears the status word (instead of
+    // a memset node before it)
     int clear_status = 0;
-    int* zero = nullptr;
-    int nzero = 0;
 };
 // out: {attempted, changed, imbalance(bits)} written to `result` (3 doubles)
 void launch_rebalance(const Grid& G, const double* work, RebalanceParams params,
