@@ -117,7 +117,15 @@ struct Grid {
 // q * extent is that zero and t - q * extent is t itself, except that a zero t
 // (of either sign) gives +0.  So the fast path is (t == 0 ? +0 : t) + lower:
 // the FP64 division, multiply and subtract are skipped without changing a bit
-// of the result.  Every other input (outside the box, NaN, inf) divides.
+// of the result.
+//
+// One box away the quotient's floor is known too.  For extent <= t < 2 extent,
+// t is at most 2 extent (1 - 2^-53), so the rounded quotient lies in
+// [1, 2 - 2^-52] and its floor is 1.  For -extent <= t < 0 the rounded
+// quotient lies in [-1, -0], and its floor is -1 unless it rounded to -0, which
+// takes |t| below extent 2^-1074 (the rule asks for 2^-500 and more).  Then
+// q * extent is extent with q's sign, exactly.  Every other input (further
+// out, NaN, inf) divides.
 //
 // With lower == 0 the fast path needs no arithmetic at all: t is v itself
 // and (t == 0 ? +0 : t) + 0 is v, or +0 for a zero of either sign.
@@ -125,6 +133,9 @@ __device__ __forceinline__ double wrap_axis(double v, double lower, double exten
     if (lower == 0.0 && v >= 0.0 && v < extent) return v == 0.0 ? 0.0 : v;
     const double t = __dsub_rn(v, lower);
     if (t >= 0.0 && t < extent) return __dadd_rn(t == 0.0 ? 0.0 : t, lower);
+    const double one = t < 0.0 ? -extent : extent;   // q * extent, one box away
+    if (t < __dadd_rn(extent, extent) && t >= -extent && (t > 0.0 || t <= __dmul_rn(extent, -0x1p-500)))
+        return __dadd_rn(__dsub_rn(t, one), lower);
     const double q = floor(__ddiv_rn(t, extent));
     return __dadd_rn(__dsub_rn(t, __dmul_rn(q, extent)), lower);
 }
