@@ -762,7 +762,7 @@ struct dsx_grid {
         work = device_alloc<double>(fixed_owned, P);
 
         const int max_tiles = static_cast<int>((ncap + dsx::kTile - 1) / dsx::kTile) + P;
-        S.stride = max_tiles + 1;
+        S.stride = (max_tiles + 4) / 4 * 4;   // a row per counter, whole groups of four
         // 30 counters per tile: the fused step's (28 halo + stays + emigrants)
         S.cnt = device_alloc<int>(fixed_owned, static_cast<std::size_t>(30) * S.stride);
         S.pre = device_alloc<int>(fixed_owned, static_cast<std::size_t>(30) * S.stride);
@@ -773,7 +773,7 @@ struct dsx_grid {
         S.imm_list = S.imm_total + P;
         S.imm_bnd = S.imm_list + static_cast<std::size_t>(P) * dsx::kMaxNeighbors;
         S.imm_img = S.imm_bnd + P;
-        S.imm_copies = dsx::immigrant_copies(P);
+        S.imm_copies = dsx::immigrant_copies(P, max_tiles);
         const std::size_t nrep = static_cast<std::size_t>(P) * (3 + dsx::kMaxNeighbors) * S.imm_copies;
         S.imm_rep = device_alloc<int>(fixed_owned, nrep);
         cuda_check(cudaMemset(S.imm_rep, 0, nrep * sizeof(int)), "memset");
@@ -784,8 +784,8 @@ struct dsx_grid {
         cuda_check(cudaMemset(S.ticket, 0, sizeof(unsigned)), "memset");
         S.imm_tiles = device_alloc<int4>(fixed_owned, static_cast<std::size_t>(max_tiles));
         S.imm_base = device_alloc<int>(fixed_owned, P);
-        S.emig_src = device_alloc<int>(fixed_owned, ncap);
-        S.emig_dst = device_alloc<int>(fixed_owned, ncap);
+        S.emig_src = device_alloc<int>(fixed_owned, static_cast<std::size_t>(ncap + 3) / 4 * 4);
+        S.emig_dst = device_alloc<int>(fixed_owned, static_cast<std::size_t>(ncap + 3) / 4 * 4);
         S.max_chunks = static_cast<int>((ncap + dsx::kTile - 1) / dsx::kTile);
         S.emig_hist = device_alloc<int>(fixed_owned, static_cast<std::size_t>(S.max_chunks) * P);
         S.emig_info = device_alloc<int>(fixed_owned, 4);
@@ -981,8 +981,7 @@ struct dsx_grid {
             dsx::launch_step_layout(G, S, stream, desc.policy != DSX_DYNAMIC);
             dsx::launch_step_bases(G, S, stream);
             dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);
-            dsx::launch_step_emigrant_list(G, S, S.imm_total, stream);
-            dsx::launch_step_emigrants(G, A, owned_off(), next_off(), S, S.imm_total, nullptr, stream);
+            dsx::launch_step_finish(G, G, A, owned_off(), next_off(), ghost_off(), S, stream, false);
         }
         commit_migrate();
         if (results) {
@@ -2814,9 +2813,9 @@ int dsx_grid_kernel_times(dsx_grid* grid, int max, const char** names, float* ms
 
 int dsx_grid_step_kernel_count(dsx_grid* grid) {
     // rebalance (Dynamic only); classify, counter scan with the layout, tile
-    // bases, move; emigrant list, histogram, column scan, placement;
-    // immigrants' classify, scan, scatter; reverse sum
-    return (grid->desc.policy == DSX_DYNAMIC ? 1 : 0) + 4 + 4 + 3 + 1;
+    // bases, move; emigrant list; histogram, column scan, placement, immigrants'
+    // classify, scan, scatter (one launch for few tiles); reverse sum
+    return (grid->desc.policy == DSX_DYNAMIC ? 1 : 0) + 4 + (dsx::few_tiles(grid->params()) ? 2 : 7) + 1;
 }
 
 }  // extern "C"

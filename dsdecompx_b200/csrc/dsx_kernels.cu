@@ -55,6 +55,45 @@ __device__ __forceinline__ int block_scan_excl(int v, int& total, int* ws) {
     return excl;
 }
 
+// K exclusive block scans at the cost of one (three barriers); totals get the
+// block sums.  ws: 33 ints of shared per value.
+template <int THREADS, int K>
+__device__ __forceinline__ void block_scans_excl(int (&v)[K], int (&total)[K], int (&ws)[K][33]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int inc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) inc[k] = v[k];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int u = __shfl_up_sync(0xffffffffu, inc[k], o);
+            if (lane >= o) inc[k] += u;
+        }
+    if (lane == 31)
+#pragma unroll
+        for (int k = 0; k < K; ++k) ws[k][warp] = inc[k];
+    __syncthreads();
+    if (warp < K) {   // warp k scans value k's warp sums
+        const int w = lane < THREADS / 32 ? ws[warp][lane] : 0;
+        int winc = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, winc, o);
+            if (lane >= o) winc += u;
+        }
+        ws[warp][lane] = winc - w;
+        if (lane == 31) ws[warp][32] = winc;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        v[k] = inc[k] - v[k] + ws[k][warp];
+        total[k] = ws[k][32];
+    }
+    __syncthreads();
+}
+
 __device__ __forceinline__ int warp_inclusive_sum(int v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -211,51 +250,75 @@ __global__ void __launch_bounds__(1024) k_scan_counters(const int* cnt, int* pre
     scan_counter(cnt, pre, stride, tile_start_end);
 }
 
+// A warp takes a run of tiles, four consecutive ones a lane and up to eight
+// rows of 128 in registers: one round trip brings the run (32,768 tiles for the
+// block), the block scans the warps' sums, and the rows are scanned and
+// written from the registers.  (One scan of five shuffles per 128 tiles: per
+// 32 the shuffles alone took 5 us of a 31,000-tile scan, all in one SM.)
 __device__ __forceinline__ void scan_counter(const int* cnt, int* pre, int stride,
                                              const int* tile_start_end) {
-    constexpr int PER = 8;
-    constexpr int CHUNK = 1024 * PER;
-    __shared__ int ws[33];
-    // a chunk of the counter, padded one word per 32 so that thread t's PER
-    // consecutive entries sit in distinct banks
-    __shared__ int buf[CHUNK + CHUNK / 32];
-    const int k = blockIdx.x;
+    constexpr int ROWS = 8;
+    __shared__ int s_sum[33];
+    const int k = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ntiles = *tile_start_end;
+    // (rows of `stride` entries, a multiple of four past the last tile's + 1)
     const int* src = cnt + static_cast<long long>(k) * stride;
     int* dst = pre + static_cast<long long>(k) * stride;
-    auto at = [](int i) { return i + (i >> 5); };
-    int carry = 0;
-    for (int base = 0; base < ntiles; base += CHUNK) {
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int i = j * 1024 + threadIdx.x;
-            buf[at(i)] = base + i < ntiles ? src[base + i] : 0;
-        }
-        __syncthreads();
-        int v[PER];
+    int before = 0;
+    for (int base = 0; base < ntiles; base += 1024 * 4 * ROWS) {
+        const int rows = min((ntiles - base + 4095) / 4096, ROWS);
+        const int begin = base + warp * rows * 128 + lane * 4;
+        int4 v[ROWS];
         int sum = 0;
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            v[j] = buf[at(threadIdx.x * PER + j)];
-            sum += v[j];
+        for (int r = 0; r < ROWS; ++r) {
+            const int i = begin + r * 128;
+            v[r] = make_int4(0, 0, 0, 0);
+            if (r < rows && i < ntiles) v[r] = *reinterpret_cast<const int4*>(src + i);
         }
-        int total;
-        int run = block_scan_excl<1024>(sum, total, ws) + carry;
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            buf[at(threadIdx.x * PER + j)] = run;
-            run += v[j];
+        for (int r = 0; r < ROWS; ++r) {
+            const int i = begin + r * 128;
+            if (i + 1 >= ntiles) v[r].y = 0;
+            if (i + 2 >= ntiles) v[r].z = 0;
+            if (i + 3 >= ntiles) v[r].w = 0;
+            sum += v[r].x + v[r].y + v[r].z + v[r].w;
+        }
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) s_sum[warp] = sum;
+        __syncthreads();
+        if (warp == 0) {
+            const int w = s_sum[lane];
+            const int incl = warp_inclusive_sum(w);
+            s_sum[lane] = incl - w;
+            if (lane == 31) s_sum[32] = incl;
         }
         __syncthreads();
+        int carry = before + s_sum[warp];
+        before += s_sum[32];
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int i = j * 1024 + threadIdx.x;
-            if (base + i < ntiles) dst[base + i] = buf[at(i)];
+        for (int r = 0; r < ROWS; ++r) {
+            if (r >= rows) break;
+            const int i = begin + r * 128;
+            const int own = v[r].x + v[r].y + v[r].z + v[r].w;
+            const int incl = warp_inclusive_sum(own);
+            int4 p;
+            p.x = carry + incl - own;
+            p.y = p.x + v[r].x;
+            p.z = p.y + v[r].y;
+            p.w = p.z + v[r].z;
+            if (i + 3 < ntiles) {
+                *reinterpret_cast<int4*>(dst + i) = p;
+            } else {
+                if (i < ntiles) dst[i] = p.x;
+                if (i + 1 < ntiles) dst[i + 1] = p.y;
+                if (i + 2 < ntiles) dst[i + 2] = p.z;
+            }
+            carry += __shfl_sync(0xffffffffu, incl, 31);
         }
-        carry += total;
-        __syncthreads();
+        __syncthreads();   // s_sum
     }
-    if (threadIdx.x == 0) dst[ntiles] = carry;
+    if (threadIdx.x == 0) dst[ntiles] = before;
 }
 
 // ----------------------------------------------------------------- migrate
@@ -1307,43 +1370,92 @@ __global__ void __launch_bounds__(1024) k_step_scan_layout(Grid G, const int* cn
     if (threadIdx.x == 0) *ticket = 0u;
 }
 
+// One CTA's latency is a small step's time (4,000 particles in 2x2x2: 12 -> 10
+// us with the scan), so the phases are few: the tile
+// sums and immigrant counters of every subdomain and list in one round trip,
+// five scans in one, the lists' lengths in shared memory for the receivers'
+// walks (kListCap lists; in global memory beyond), and the counters' bases
+// written where a list's first slot is found.
+constexpr int kListCap = 256 * kMaxNeighbors;
+
 __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, int stride,
                                                  const StepTables& T) {
-    __shared__ int ws[33];
-    __shared__ int s_rcv[kMaxRanks + 1];
+    __shared__ int ws[5][33];
+    __shared__ int s_rcv[kMaxRanks];
     __shared__ int s_snd[kMaxRanks];
-    __shared__ int s_ts[kMaxRanks + 1];   // the current layout's tile starts, staged once
-    const int P = G.P;
+    __shared__ int s_ts[kMaxRanks + 1];   // the current layout's tile starts
+    __shared__ int s_len[kListCap];
+    const int P = G.P, lists = P * kMaxNeighbors;
     const int t = threadIdx.x;
+    const int warp = t >> 5, lane = t & 31, nwarps = blockDim.x >> 5;
+    int* len_of = lists <= kListCap ? s_len : T.list_len;
     for (int k = t; k <= P; k += blockDim.x) s_ts[k] = G.tile_start[k];
     __syncthreads();
     const int ntiles = s_ts[P];
-    const int* ts_old = s_ts;
     auto tile_sum = [&](int k, int r) {
-        return __ldcg(pre + k * stride + ts_old[r + 1]) - __ldcg(pre + k * stride + ts_old[r]);
+        return __ldcg(pre + k * stride + s_ts[r + 1]) - __ldcg(pre + k * stride + s_ts[r]);
     };
-    sum_immigrants(P, T.imm_total, T.imm_rep, T.copies);
-    unsigned status = 0;
-    // new owned layout and migration results
-    int retained = 0, received = 0, old = 0, next = 0;
+    const int copies = T.copies, block = kImmCounters * P;
+    // an immigrant counter: its copies summed and left zero for the next step
+    auto immigrants = [&](int at) {
+        int sum = 0;
+#pragma unroll 16
+        for (int c = 0; c < copies; ++c) sum += __ldcg(T.imm_rep + static_cast<long long>(c) * block + at);
+        for (int c = 0; c < copies; ++c) T.imm_rep[static_cast<long long>(c) * block + at] = 0;
+        return sum;
+    };
+    // send-list lengths: retained part from the tile prefixes, immigrant part
+    // from the classify's counters
+    for (int idx = t; idx < lists; idx += blockDim.x) {
+        const int r = idx / kMaxNeighbors, n = idx % kMaxNeighbors;
+        const bool active = G.need[r * 32 + n] & 64;
+        const int imm = immigrants(P + idx);
+        const int ret = active ? tile_sum(n, r) : 0;
+        const int len = active ? ret + imm : 0;
+        T.imm_list[idx] = imm;
+        T.list_ret[idx] = ret;
+        T.list_len[idx] = len;
+        len_of[idx] = len;
+        if (!active) {
+            T.cbase_ret[r * kHaloCounters + n] = 0;
+            T.cbase_imm[r * kHaloCounters + n] = 0;
+        }
+    }
+    // per subdomain: the next owned layout, boundary owners and images (the
+    // retained part first, then the immigrants)
+    int retained = 0, received = 0, old = 0, bret = 0, iret = 0;
+    int v[5] = {0, 0, 0, 0, 0}, total[5];   // next count, its tiles, immigrant tiles, owners, images
     if (t < P) {
         retained = tile_sum(kStepStay, t);
-        received = T.imm_total[t];
+        received = immigrants(t);
         old = G.n[t];
-        next = retained + received;
+        bret = tile_sum(kBoundaryCounter, t);
+        iret = tile_sum(kImageCounter, t);
+        const int bimm = immigrants((1 + kMaxNeighbors) * P + t);
+        const int iimm = immigrants((2 + kMaxNeighbors) * P + t);
+        T.imm_total[t] = received;
+        T.imm_bnd[t] = bimm;
+        T.imm_img[t] = iimm;
+        v[0] = retained + received;
+        v[1] = (v[0] + G.tile - 1) / G.tile;
+        v[2] = (received + G.tile - 1) / G.tile;
+        v[3] = bret + bimm;
+        v[4] = iret + iimm;
     }
-    int total_next, total_tiles, total_imm_tiles;
-    const int ob = block_scan_excl<1024>(next, total_next, ws);
-    const int ntl = t < P ? (next + G.tile - 1) / G.tile : 0;
-    const int ts = block_scan_excl<1024>(ntl, total_tiles, ws);
-    const int itl = t < P ? (received + G.tile - 1) / G.tile : 0;
-    const int its = block_scan_excl<1024>(itl, total_imm_tiles, ws);
+    const int next = v[0];
+    block_scans_excl<1024, 5>(v, total, ws);   // (its barriers complete len_of)
     if (t < P) {
         G.n_next[t] = next;
-        G.obase_next[t] = ob;
-        G.tile_start_next[t] = ts;
-        T.imm_base[t] = ob + retained;
-        T.imm_tile_start[t] = its;
+        G.obase_next[t] = v[0];
+        G.tile_start_next[t] = v[1];
+        T.imm_base[t] = v[0] + retained;
+        T.imm_tile_start[t] = v[2];
+        int* cr = T.cbase_ret + t * kHaloCounters;
+        int* ci = T.cbase_imm + t * kHaloCounters;
+        cr[kBoundaryCounter] = v[3];
+        ci[kBoundaryCounter] = v[3] + bret;
+        cr[kImageCounter] = v[4];
+        ci[kImageCounter] = v[4] + iret;
         long long* o = T.results + 6 * t;
         o[1] = old;
         o[2] = retained;
@@ -1352,98 +1464,56 @@ __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, 
         o[5] = next;
         o[0] = (o[3] != 0 || o[4] != 0) ? 1 : 0;
     }
+    // receivers and senders, one warp each (lane m: the block of neighbor m)
+    for (int q = warp; q < P; q += nwarps) {
+        const int e = lane < kMaxNeighbors ? ro(G.sender_of + q * kMaxNeighbors + lane) : -1;
+        const int got = __reduce_add_sync(0xffffffffu, e >= 0 ? len_of[e] : 0);
+        const int sent = __reduce_add_sync(0xffffffffu, lane < kMaxNeighbors ? len_of[q * kMaxNeighbors + lane] : 0);
+        if (lane == 0) {
+            s_rcv[q] = got;
+            s_snd[q] = sent;
+        }
+    }
+    __syncthreads();
+    int u[2] = {t < P ? s_rcv[t] : 0, t < P ? s_snd[t] : 0}, ghosts[2];
+    const int mine = u[0];
+    __shared__ int ws2[2][33];
+    block_scans_excl<1024, 2>(u, ghosts, ws2);
+    if (t < P) {
+        T.gq[t] = mine;
+        T.gbase[t] = u[0];
+        s_rcv[t] = u[0];
+        s_snd[t] = u[1];
+    }
+    __syncthreads();
+    for (int q = warp; q < P; q += nwarps) {
+        // the lists toward q, in q's neighbor order: their first slots, and
+        // the bases of their senders' counters
+        const int e = lane < kMaxNeighbors ? ro(G.sender_of + q * kMaxNeighbors + lane) : -1;
+        const int len = e >= 0 ? len_of[e] : 0;
+        const int slot = s_rcv[q] + warp_inclusive_sum(len) - len;
+        if (e >= 0) {
+            const int r = e / kMaxNeighbors, n = e % kMaxNeighbors;
+            T.send_base[e] = slot;
+            T.cbase_ret[r * kHaloCounters + n] = slot;
+            T.cbase_imm[r * kHaloCounters + n] = slot + T.list_ret[e];
+        }
+        write_list_flat(len_of, T.list_flat, q, s_snd[q]);
+    }
     if (t == 0) {
-        G.obase_next[P] = total_next;
-        G.tile_start_next[P] = total_tiles;
-        T.imm_tile_start[P] = total_imm_tiles;
+        unsigned status = 0;
+        G.obase_next[P] = total[0];
+        G.tile_start_next[P] = total[1];
+        T.imm_tile_start[P] = total[2];
         const int E = __ldcg(pre + kStepEmig * stride + ntiles);
         T.emig_info[0] = E;
         T.emig_info[1] = (E + TILE - 1) / TILE;
-        if (total_next != G.obase[P]) status |= kStatusMigrationMismatch;
-    }
-    // send-list lengths: retained part from the tile prefixes, immigrant part
-    // from the atomics of F1
-    for (int idx = t; idx < P * kMaxNeighbors; idx += blockDim.x) {
-        const int r = idx / kMaxNeighbors, n = idx % kMaxNeighbors;
-        const bool active = n < G.nn[r] && G.nbr[idx] >= 0;
-        const int ret = active ? tile_sum(n, r) : 0;
-        T.list_ret[idx] = ret;
-        T.list_len[idx] = active ? ret + T.imm_list[idx] : 0;
-    }
-    __syncthreads();
-    // (the tile descriptors of the next layout and of the immigrant segments
-    // are written by k_tile_bases, over the whole grid)
-    // receivers: blocks in the receiver's neighbor order, one warp per
-    // receiver (lane m reads the block of neighbor m)
-    const int warp = t >> 5, lane = t & 31, nwarps = blockDim.x >> 5;
-    for (int q = warp; q < P; q += nwarps) {
-        int len = 0;
-        if (lane < G.nn[q]) {
-            const int e = G.sender_of[q * kMaxNeighbors + lane];
-            len = e >= 0 ? T.list_len[e] : 0;
-        }
-        const int sum = __reduce_add_sync(0xffffffffu, len);
-        const int sent = lane < kMaxNeighbors ? T.list_len[q * kMaxNeighbors + lane] : 0;
-        const int out = __reduce_add_sync(0xffffffffu, sent);
-        if (lane == 0) {
-            s_rcv[q] = sum;
-            s_snd[q] = out;
-        }
-    }
-    __syncthreads();
-    const int mine = t < P ? s_rcv[t] : 0;
-    const int sent_all = t < P ? s_snd[t] : 0;
-    int total_ghosts, total_sent;
-    const int gb = block_scan_excl<1024>(mine, total_ghosts, ws);
-    const int sb = block_scan_excl<1024>(sent_all, total_sent, ws);
-    if (t < P) {
-        T.gq[t] = mine;
-        T.gbase[t] = gb;
-        s_rcv[t] = gb;
-        s_snd[t] = sb;
-    }
-    __syncthreads();
-    for (int q = warp; q < P; q += nwarps) {
-        write_list_flat(T.list_len, T.list_flat, q, s_snd[q]);
-        int len = 0, e = -1;
-        if (lane < G.nn[q]) {
-            e = G.sender_of[q * kMaxNeighbors + lane];
-            len = e >= 0 ? T.list_len[e] : 0;
-        }
-        const int incl = warp_inclusive_sum(len);
-        if (e >= 0) T.send_base[e] = s_rcv[q] + incl - len;
-    }
-    // boundary owners and images: retained part first, then the immigrants
-    int bret = 0, bimm = 0, iret = 0, iimm = 0;
-    if (t < P) {
-        bret = tile_sum(kBoundaryCounter, t);
-        bimm = T.imm_bnd[t];
-        iret = tile_sum(kImageCounter, t);
-        iimm = T.imm_img[t];
-    }
-    int total_b, total_i;
-    const int bb = block_scan_excl<1024>(bret + bimm, total_b, ws);
-    const int ib = block_scan_excl<1024>(iret + iimm, total_i, ws);   // syncs: send_base complete
-    for (int e = t; e < P * kMaxNeighbors; e += blockDim.x) {
-        const int r = e / kMaxNeighbors, n = e % kMaxNeighbors;
-        const bool active = n < G.nn[r] && G.nbr[e] >= 0;
-        T.cbase_ret[r * kHaloCounters + n] = active ? T.send_base[e] : 0;
-        T.cbase_imm[r * kHaloCounters + n] = active ? T.send_base[e] + T.list_ret[e] : 0;
-    }
-    if (t < P) {
-        int* cr = T.cbase_ret + t * kHaloCounters;
-        int* ci = T.cbase_imm + t * kHaloCounters;
-        cr[kBoundaryCounter] = bb;
-        ci[kBoundaryCounter] = bb + bret;
-        cr[kImageCounter] = ib;
-        ci[kImageCounter] = ib + iret;
-    }
-    if (t == 0) {
-        T.gbase[P] = total_ghosts;
-        T.info[0] = total_ghosts;
-        T.info[1] = total_b;
-        if (static_cast<long long>(total_ghosts) > G.gcap) status |= kStatusGhostOverflow;
-        else T.boff[total_b] = total_i;
+        if (total[0] != G.obase[P]) status |= kStatusMigrationMismatch;
+        T.gbase[P] = ghosts[0];
+        T.info[0] = ghosts[0];
+        T.info[1] = total[3];
+        if (static_cast<long long>(ghosts[0]) > G.gcap) status |= kStatusGhostOverflow;
+        else T.boff[total[3]] = total[4];
         if (T.fresh_status) *G.status = status;
         else if (status) atomicOr(G.status, status);
     }
@@ -2337,6 +2407,143 @@ __global__ void __launch_bounds__(NT) k_emig_list(Grid G, const int* pre, int st
     }
     fill_tiles_grid(G.P, G.tile, G.n_next, G.obase_next, G.tile_start_next, G.tiles_next);
     fill_tiles_grid(G.P, G.tile, imm_in, imm_base, imm_ts, imm_tiles);
+}
+
+// The emigrants' chain after their list in one launch, for grids of few tiles:
+// one CTA per destination picks its immigrants from the list (in its order),
+// writes their records after the retained ones, and their ghost images and
+// CSR entries after the retained parts of the send lists -- what k_emig_hist,
+// k_emig_colscan, k_emig_place and the immigrants' k_halo_classify,
+// k_scan_counters and k_halo_scatter do in six launches of some 4 us each,
+// whose latency is a small step's time.  Every CTA reads the whole list, so its
+// time grows with the emigrants: 262,000 particles (1,400 leavers) 11 us against
+// 27 for the chain, 500,000 (3,000) 21, beside a move of 26; beyond 1,024 tiles
+// (kImmigrantTiles) the chain, whose time does not grow, is hidden behind the
+// move.
+//
+// order: [ncap] scratch, the source of every immigrant by its new slot.
+constexpr int kImmThreads = 512;
+constexpr int kImmWarps = kImmThreads / 32;
+
+__global__ void __launch_bounds__(kImmThreads, 1) k_step_immigrants(
+    Grid G, Arrays A, long long src_off, long long dst_off, long long ghost_off, const int* emig_info,
+    const int* __restrict__ emig_src, const int* __restrict__ emig_dst, const int* imm_total,
+    const int* imm_base, const int* cbase_imm, int* order, MoveOutputs O) {
+    pdl_begin();
+    __shared__ int ws[33];
+    __shared__ int s_cnt[kImmWarps][32];
+    __shared__ int s_run[32];
+    const int d = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lt = lanemask_lt();
+    const int base = imm_base[d], expected = imm_total[d];
+    const bool ghosts = !(*G.status & kStatusGhostOverflow);
+    if (threadIdx.x < kHaloCounters) s_run[threadIdx.x] = cbase_imm[d * kHaloCounters + threadIdx.x];
+    // the immigrants' sources, in the list's order, four entries a thread
+    const int E = emig_info[0];
+    int n = 0;
+    for (int e0 = 0; e0 < E; e0 += 4 * kImmThreads) {
+        const int e = e0 + 4 * threadIdx.x;
+        int4 to = make_int4(-1, -1, -1, -1), from = make_int4(0, 0, 0, 0);
+        if (e < E) {   // (the list's storage is whole groups of four)
+            to = ro(reinterpret_cast<const int4*>(emig_dst + e));
+            from = ro(reinterpret_cast<const int4*>(emig_src + e));
+        }
+        const bool m0 = to.x == d, m1 = to.y == d && e + 1 < E, m2 = to.z == d && e + 2 < E,
+                   m3 = to.w == d && e + 3 < E;
+        int total;
+        int at = base + n + block_scan_excl<kImmThreads>(m0 + m1 + m2 + m3, total, ws);
+        n += total;
+        // past the layout's count only after a mismatch, which is reported
+        if (n <= expected) {
+            if (m0) order[at++] = from.x;
+            if (m1) order[at++] = from.y;
+            if (m2) order[at++] = from.z;
+            if (m3) order[at] = from.w;
+        }
+    }
+    if (threadIdx.x == 0 && n != expected) atomicOr(G.status, kStatusMigrationMismatch);
+    if (n > expected) n = expected;
+    __syncthreads();   // the order, written by every thread
+    const TileBounds bounds = halo_bounds(G, d);
+    const ListTest list = list_test(G, d, lane);
+    const double* shift = G.shift + static_cast<long long>(d) * kMaxNeighbors * 3;
+    for (int r0 = 0; r0 < n; r0 += kImmThreads) {
+        const int r = r0 + threadIdx.x;
+        const bool in = r < n;
+        const int ni = base + r;
+        long long src = 0;
+        unsigned flags = 0;
+        double v[11] = {};
+        int ty = 0, id = 0;
+        if (in) {
+            src = src_off + order[ni];
+#pragma unroll
+            for (int a = 0; a < 11; ++a) v[a] = ro(A.d[a] + src);
+            ty = ro(A.type + src);
+            id = ro(A.gid + src);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) v[a] = wrap_if(G, a, v[a]);
+            if (ghosts) flags = halo_flags(bounds, v[0], v[1], v[2]);
+            const long long to = dst_off + ni;
+#pragma unroll
+            for (int a = 0; a < 11; ++a) A.d[a][to] = v[a];
+            A.type[to] = ty;
+            A.gid[to] = id;
+            copy_fields(A.f, src, to);
+        }
+        if (!ghosts) continue;
+        unsigned w[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) w[k] = __ballot_sync(0xffffffffu, (flags >> k) & 1u);
+        const unsigned members = list_members(list, w);
+        const unsigned any = __reduce_or_sync(0xffffffffu, members);
+        unsigned m = (any >> lane) & 1u ? ro(G.lut + d * 64 + flags) : 0u;
+        const int acc = __popc(members);
+        const int images = __reduce_add_sync(0xffffffffu, acc);
+        s_cnt[warp][lane] = lane == kBoundaryCounter ? __popc(any) : lane == kImageCounter ? images : acc;
+        __syncthreads();
+        int run = lane < kHaloCounters ? s_run[lane] : 0, all = 0;
+        for (int k = 0; k < kImmWarps; ++k) {
+            const int c = s_cnt[k][lane];
+            run += k < warp ? c : 0;
+            all += c;
+        }
+        __syncthreads();
+        if (warp == 0 && lane < kHaloCounters) s_run[lane] += all;
+        if (any) {
+            const int b = __shfl_sync(0xffffffffu, run, kBoundaryCounter) + __popc(any & lt);
+            const int pm = __popc(m);
+            int img = __shfl_sync(0xffffffffu, run, kImageCounter) + warp_inclusive_sum(pm) - pm;
+            if (pm) {
+                O.bowner[b] = ni;
+                O.boff[b] = img;
+            }
+            bool first = true;
+            while (__any_sync(0xffffffffu, m != 0)) {
+                const int k = m ? __ffs(m) - 1 : 0;
+                const unsigned its = __shfl_sync(0xffffffffu, members, k);
+                const int slot = __shfl_sync(0xffffffffu, run, k) + __popc(its & lt);
+                if (m) {
+                    O.bslot[img++] = slot;
+                    if (first) O.bfirst[b] = slot;
+                    first = false;
+                    const long long gi = ghost_off + slot;
+#pragma unroll
+                    for (int a = 0; a < 11; ++a)
+                        A.d[a][gi] = a < 3 ? __dadd_rn(v[a], ro(shift + 3 * k + a))
+                                           : a < 6 || a > 8 ? v[a] : 0.0;
+                    A.type[gi] = ty;
+                    A.gid[gi] = id;
+                    copy_fields(A.f, src, gi);
+                    O.ghost_owner[slot] = ni;
+                    O.ghost_entry[slot] = d * kMaxNeighbors + k;
+                    m &= m - 1;
+                }
+            }
+        }
+        __syncthreads();   // s_run moved on before the next pass reads it
+    }
 }
 
 // The tile prefixes of the step's counters summed per subdomain, for a
@@ -3696,7 +3903,11 @@ bool staged_passes(const Arrays& A, int* ends, int& passes) {
     return true;
 }
 
-int immigrant_copies(int P) { return P >= 256 ? 1 : P >= 8 ? 256 / P : 32; }
+int immigrant_copies(int P, int max_tiles) {
+    const int most = P >= 256 ? 1 : P >= 8 ? 256 / P : 32;
+    const int wanted = max_tiles / 512;
+    return wanted < 1 ? 1 : wanted < most ? wanted : most;
+}
 
 void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, const Scratch& S,
                           cudaStream_t s, bool clear_counters) {
@@ -3813,11 +4024,25 @@ void launch_step_export(const Grid& G, const Scratch& S, int* out, cudaStream_t 
     pdl_launch(k_step_export, 1, 1024, 0, s, G, S.pre, S.stride, out, S.imm_total, S.imm_rep, S.imm_copies);
 }
 
+// Up to this many tiles one CTA per destination handles the emigrants
+// (k_step_immigrants, where the sizes behind the line stand).
+constexpr int kImmigrantTiles = 1024;
+
+bool few_tiles(const Grid& G) { return G.max_tiles <= kImmigrantTiles; }
+
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
-                        long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s) {
+                        long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s,
+                        bool halo) {
     launch_step_emigrant_list(G, S, S.imm_total, s);
+    if (few_tiles(G)) {
+        const MoveOutputs O{S.ghost_owner, S.ghost_entry, S.bowner, S.boff, S.bslot, S.bfirst};
+        pdl_launch(k_step_immigrants, G.P, kImmThreads, 0, s, G, A, src_off, dst_off, ghost_off, S.emig_info,
+                   S.emig_src, S.emig_dst, S.imm_total, S.imm_base, S.cbase_imm,
+                   reinterpret_cast<int*>(S.mask), O);
+        return;
+    }
     launch_step_emigrants(G, A, src_off, dst_off, S, S.imm_total, nullptr, s);
-    launch_step_immigrant_halo(Gn, A, dst_off, ghost_off, S, s);
+    if (halo) launch_step_immigrant_halo(Gn, A, dst_off, ghost_off, S, s);
 }
 
 void launch_step_immigrant_halo(const Grid& Gn, const Arrays& A, long long dst_off,

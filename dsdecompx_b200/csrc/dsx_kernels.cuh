@@ -139,16 +139,21 @@ cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, lo
 void launch_step_classify(const Grid& G, const Arrays& A, long long src_off, const Scratch& S,
                           cudaStream_t s, bool clear_counters = false);
 void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s, bool fresh_status = false);
-// Copies of the immigrant counters for P subdomains: 256 counters' worth of
-// addresses for each sum where P is small (the layout reads every copy).
-int immigrant_copies(int P);
+// Copies of the immigrant counters: 256 addresses for each kind of sum where P
+// is small, one copy per 512 tiles at most (a small grid's few leavers do not
+// wait for each other, and the layout reads every copy).
+int immigrant_copies(int P, int max_tiles);
 void launch_step_bases(const Grid& G, const Scratch& S, cudaStream_t s);
 // imm_in: immigrants per subdomain whose ghost images this grid makes
 void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s);
 void launch_step_move(const Grid& G, const Arrays& A, long long src_off, long long dst_off,
                       long long ghost_off, const Scratch& S, cudaStream_t s);
+// halo false: a migrate alone (its grid's halo table is empty).
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
-                        long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s);
+                        long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s,
+                        bool halo = true);
+// The finish is two launches (few tiles) instead of seven.
+bool few_tiles(const Grid& G);
 // The finish in its two parts: the emigrants' stable multi-split into the
 // next half (local_imm: emigrants expected per destination, checked; gap:
 // null, or P x P slots left before each source's group for other shards'

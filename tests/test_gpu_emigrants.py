@@ -1,0 +1,52 @@
+"""Both ways of placing emigrants (one CTA per destination up to 1,024 tiles,
+the chain of kernels beyond) and the counters around them, against the oracle:
+list lengths around the four entries a thread reads, more immigrants than one
+pass of a CTA takes, tile counts around the scan's rows, and few enough
+subdomains for copies of the immigrant counters."""
+import numpy as np
+import pytest
+
+from helpers import Pair, split_by_owner, uniform_particles
+
+pytestmark = pytest.mark.gpu
+
+
+def check(pair, rng, sigma, steps=2):
+    import torch
+
+    stream = torch.cuda.Stream()
+    for step in range(steps):
+        pair.displace(rng, sigma)
+        torch.cuda.synchronize()
+        if step:      # the batched step, then the calls it stands for
+            assert pair.gpu.step(capture=True, stream=stream) == 0
+            pair.ref.migrate()
+            pair.ref.exchange_halo(rebuild=True)
+            pair.ref.reverse_halo()
+        else:
+            assert (pair.gpu.migrate() == pair.ref.migrate()).all()
+            hg, hr = pair.gpu.exchange_halo(rebuild=True), pair.ref.exchange_halo(rebuild=True)
+            assert (hg[:, 0] == hr[:, 0]).all()
+        pair.compare(f"step {step}")
+
+
+@pytest.mark.parametrize("dims,n,sigma", [
+    ((2, 1, 1), 7, 0.6),             # a list shorter than one thread's entries
+    ((5, 1, 1), 2_049, 0.02),        # a few emigrants
+    ((2, 2, 2), 4_097, 3.0),         # most leave: a destination's passes and list passes
+    ((3, 2, 2), 40_000, 0.3),
+    ((2, 1, 2), 530_000, 0.2),       # more than 1,024 tiles: the chain, two counter copies
+], ids=["tiny", "few", "most", "mid", "chain"])
+def test_emigrants_follow_the_oracle(cuda, dims, n, sigma):
+    rng = np.random.default_rng(n)
+    fields = [("q", "float64", 1), ("v", "float32", 3)] if n < 100_000 else []
+    L = [4.0 * d for d in dims]
+    pair = Pair(int(np.prod(dims)), dims, "manual", (0, 0, 0), L, (True, True, True), 0.5, True,
+                None, fields, particles=n, ghost_capacity=3 * n + 1000)
+    try:
+        data = uniform_particles(rng, n, (0, 0, 0), L, fields)
+        owner = pair.ref.owner_rank(np.stack([data["x"], data["y"], data["z"]], 1))
+        pair.upload(split_by_owner(owner, data, pair.P))
+        check(pair, rng, sigma)
+    finally:
+        pair.close()
