@@ -809,88 +809,95 @@ __device__ __forceinline__ void write_list_flat(const int* list_len, int* list_f
     if (lane < kMaxNeighbors) list_flat[r * kMaxNeighbors + lane] = first + incl - len;
 }
 
-// S2b: send-list lengths, receiver ghost layout (blocks in the receiver's
-// neighbor order, dsDecompX src/halo.cpp:609-649) and the first ghost slot of
-// every send list.  One CTA, one thread per receiver.
-__global__ void __launch_bounds__(1024) k_halo_layout(Grid G, const int* pre, int stride,
-                                                       int* list_len, int* send_base,
-                                                       int* list_flat, int* gq, int* gbase,
-                                                       int* boff, int* info, int* cbase) {
+// Lists whose lengths a layout keeps in shared memory.
+constexpr int kListCap = 256 * kMaxNeighbors;
+
+// S2b: the counter scan and, in the CTA that finishes last (as in
+// k_step_scan_layout), the send-list lengths, the receiver ghost layout (blocks
+// in the receiver's neighbor order, dsDecompX src/halo.cpp:609-649), the first
+// ghost slot of every send list, and per subdomain and counter the value that
+// turns a tile prefix into the global index (first slot of each send list,
+// boundary and image prefixes).
+__global__ void __launch_bounds__(1024) k_halo_scan_layout(Grid G, const int* cnt, int* pre,
+                                                            int stride, int* list_len,
+                                                            int* send_base, int* list_flat, int* gq,
+                                                            int* gbase, int* boff, int* info,
+                                                            int* cbase, unsigned* ticket) {
     pdl_begin();
-    __shared__ int ws[33];
-    __shared__ int s_rcv[kMaxRanks + 1];
+    __shared__ bool s_last;
+    scan_counter(cnt, pre, stride, G.tile_start + G.P);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    __shared__ int ws[2][33];
+    __shared__ int s_rcv[kMaxRanks];
     __shared__ int s_snd[kMaxRanks];
-    const int P = G.P;
-    const int ntiles = G.tile_start[P];
-    for (int idx = threadIdx.x; idx < P * kMaxNeighbors; idx += blockDim.x) {
+    __shared__ int s_ts[kMaxRanks + 1];
+    __shared__ int s_len[kListCap];
+    const int P = G.P, lists = P * kMaxNeighbors;
+    const int t = threadIdx.x;
+    const int warp = t >> 5, lane = t & 31, nwarps = blockDim.x >> 5;
+    int* len_of = lists <= kListCap ? s_len : list_len;
+    for (int k = t; k <= P; k += blockDim.x) s_ts[k] = G.tile_start[k];
+    __syncthreads();
+    const int ntiles = s_ts[P];
+    for (int idx = t; idx < lists; idx += blockDim.x) {
         const int r = idx / kMaxNeighbors, n = idx % kMaxNeighbors;
-        int len = 0;
-        if (n < G.nn[r] && G.nbr[idx] >= 0)
-            len = pre[n * stride + G.tile_start[r + 1]] - pre[n * stride + G.tile_start[r]];
+        const bool active = G.need[r * 32 + n] & 64;
+        const int len = active ? __ldcg(pre + n * stride + s_ts[r + 1]) - __ldcg(pre + n * stride + s_ts[r]) : 0;
         list_len[idx] = len;
+        len_of[idx] = len;
+        if (!active) cbase[r * kHaloCounters + n] = 0;
+    }
+    if (t < P) {
+        cbase[t * kHaloCounters + kBoundaryCounter] = __ldcg(pre + kBoundaryCounter * stride + s_ts[t]);
+        cbase[t * kHaloCounters + kImageCounter] = __ldcg(pre + kImageCounter * stride + s_ts[t]);
     }
     __syncthreads();
-    // receivers, one warp each: lane m reads the block of neighbor m
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    // receivers and senders, one warp each (lane m: the block of neighbor m)
     for (int r = warp; r < P; r += nwarps) {
-        int len = 0;
-        if (lane < G.nn[r]) {
-            const int e = G.sender_of[r * kMaxNeighbors + lane];
-            len = e >= 0 ? list_len[e] : 0;
-        }
-        const int sum = __reduce_add_sync(0xffffffffu, len);
-        const int sent = lane < kMaxNeighbors ? list_len[r * kMaxNeighbors + lane] : 0;
-        const int out = __reduce_add_sync(0xffffffffu, sent);
+        const int e = lane < kMaxNeighbors ? ro(G.sender_of + r * kMaxNeighbors + lane) : -1;
+        const int got = __reduce_add_sync(0xffffffffu, e >= 0 ? len_of[e] : 0);
+        const int sent = __reduce_add_sync(0xffffffffu, lane < kMaxNeighbors ? len_of[r * kMaxNeighbors + lane] : 0);
         if (lane == 0) {
-            s_rcv[r] = sum;
-            s_snd[r] = out;
+            s_rcv[r] = got;
+            s_snd[r] = sent;
         }
     }
     __syncthreads();
-    const int q = threadIdx.x;
-    const int mine = q < P ? s_rcv[q] : 0;
-    const int sent_all = q < P ? s_snd[q] : 0;
-    int total, total_sent;
-    const int excl = block_scan_excl<1024>(mine, total, ws);
-    const int sent_excl = block_scan_excl<1024>(sent_all, total_sent, ws);
-    if (q < P) {
-        gq[q] = mine;
-        gbase[q] = excl;
-        s_rcv[q] = excl;
-        s_snd[q] = sent_excl;
+    int u[2] = {t < P ? s_rcv[t] : 0, t < P ? s_snd[t] : 0}, total[2];
+    const int mine = u[0];
+    block_scans_excl<1024, 2>(u, total, ws);
+    if (t < P) {
+        gq[t] = mine;
+        gbase[t] = u[0];
+        s_rcv[t] = u[0];
+        s_snd[t] = u[1];
     }
     __syncthreads();
     for (int r = warp; r < P; r += nwarps) {
-        write_list_flat(list_len, list_flat, r, s_snd[r]);
-        int len = 0, e = -1;
-        if (lane < G.nn[r]) {
-            e = G.sender_of[r * kMaxNeighbors + lane];
-            len = e >= 0 ? list_len[e] : 0;
+        const int e = lane < kMaxNeighbors ? ro(G.sender_of + r * kMaxNeighbors + lane) : -1;
+        const int len = e >= 0 ? len_of[e] : 0;
+        const int slot = s_rcv[r] + warp_inclusive_sum(len) - len;
+        if (e >= 0) {
+            send_base[e] = slot;
+            cbase[e / kMaxNeighbors * kHaloCounters + e % kMaxNeighbors] = slot;
         }
-        const int incl = warp_inclusive_sum(len);
-        if (e >= 0) send_base[e] = s_rcv[r] + incl - len;
+        write_list_flat(len_of, list_flat, r, s_snd[r]);
     }
-    if (q == 0) {
-        gbase[P] = total;
-        const int B = pre[kBoundaryCounter * stride + ntiles];
-        const int images = pre[kImageCounter * stride + ntiles];
-        info[0] = total;
+    if (t == 0) {
+        gbase[P] = total[0];
+        const int B = __ldcg(pre + kBoundaryCounter * stride + ntiles);
+        info[0] = total[0];
         info[1] = B;
-        if (static_cast<long long>(total) > G.gcap) {
-            atomicOr(G.status, kStatusGhostOverflow);
-        } else {
-            boff[B] = images;
-        }
-    }
-    __syncthreads();
-    // per subdomain and counter, the value that turns a tile prefix into the
-    // global index: first slot of each send list, boundary/image prefixes
-    for (int idx = threadIdx.x; idx < P * kHaloCounters; idx += blockDim.x) {
-        const int r = idx / kHaloCounters, k = idx % kHaloCounters;
-        int v;
-        if (k < kMaxNeighbors) v = (k < G.nn[r] && G.nbr[r * kMaxNeighbors + k] >= 0) ? send_base[r * kMaxNeighbors + k] : 0;
-        else v = pre[k * stride + G.tile_start[r]];
-        cbase[idx] = v;
+        if (static_cast<long long>(total[0]) > G.gcap) atomicOr(G.status, kStatusGhostOverflow);
+        else boff[B] = __ldcg(pre + kImageCounter * stride + ntiles);
+        *ticket = 0u;
     }
 }
 
@@ -1317,6 +1324,72 @@ __global__ void __launch_bounds__(CT, MINB) k_step_classify(Grid G, const double
     }
 }
 
+// H1 of a per-call plan build: the bits of every owned particle at its present
+// owner ("stays": every particle of the tile) and the tile's list counters, in
+// the words and the counting of k_step_classify (1M particles: 14 us with a
+// mask per particle, 8 so).
+constexpr int kBitsThreads = 128;
+
+__global__ void __launch_bounds__(kBitsThreads, 8) k_halo_bits(Grid G, const double* __restrict__ x,
+                                                               const double* __restrict__ y,
+                                                               const double* __restrict__ z, int* cnt,
+                                                               int stride,
+                                                               unsigned* __restrict__ bits_out) {
+    pdl_begin();
+    constexpr int CI = TILE / kBitsThreads, CW = kBitsThreads / 32;
+    __shared__ int s_cnt[CW][32];
+    const int g = blockIdx.x;
+    const int4 td = G.tiles[g];   // (a row for every block of the launch)
+    if (g >= G.tile_start[G.P]) return;
+    const int s = td.x, begin = td.y, end = td.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wbegin = begin + warp * 32 * CI;
+    double px[CI], py[CI], pz[CI];
+#pragma unroll
+    for (int j = 0; j < CI; ++j) {
+        const int i = wbegin + j * 32 + lane;
+        if (i < end) {
+            px[j] = ro(x + i);
+            py[j] = ro(y + i);
+            pz[j] = ro(z + i);
+        }
+    }
+    const TileBounds bs = halo_bounds(G, s);
+    const ListTest list = list_test(G, s, lane);
+    int acc = 0, boundary = 0;
+#pragma unroll
+    for (int j = 0; j < CI; ++j) {
+        const bool valid = wbegin + j * 32 + lane < end;
+        unsigned w[kGroupWords];
+        w[0] = __ballot_sync(0xffffffffu, valid && px[j] < bs.lo[0]);
+        w[1] = __ballot_sync(0xffffffffu, valid && px[j] > bs.hi[0]);
+        w[2] = __ballot_sync(0xffffffffu, valid && py[j] < bs.lo[1]);
+        w[3] = __ballot_sync(0xffffffffu, valid && py[j] > bs.hi[1]);
+        w[4] = __ballot_sync(0xffffffffu, valid && pz[j] < bs.lo[2]);
+        w[5] = __ballot_sync(0xffffffffu, valid && pz[j] > bs.hi[2]);
+        w[6] = __ballot_sync(0xffffffffu, valid);
+        w[7] = 0u;
+        if (lane == 0) {
+            uint4* out = reinterpret_cast<uint4*>(bits_out + static_cast<long long>(g) * kTileWords +
+                                                  (warp * CI + j) * kGroupWords);
+            out[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            out[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+        const unsigned six[6] = {w[0], w[1], w[2], w[3], w[4], w[5]};
+        const unsigned members = list_members(list, six);
+        acc += __popc(members);
+        boundary += __popc(__reduce_or_sync(0xffffffffu, members));
+    }
+    const int images = __reduce_add_sync(0xffffffffu, acc);
+    s_cnt[warp][lane] = lane == kBoundaryCounter ? boundary : lane == kImageCounter ? images : acc;
+    __syncthreads();
+    if (threadIdx.x < kHaloCounters) {
+        int sum = 0;
+        for (int w = 0; w < CW; ++w) sum += s_cnt[w][threadIdx.x];
+        cnt[threadIdx.x * stride + g] = sum;
+    }
+}
+
 // F3: the new owned layout, the ghost layout of the whole plan (retained +
 // immigrant parts of every send list), the CSR bases and the immigrant
 // segments.  One CTA, one thread per subdomain.
@@ -1376,7 +1449,6 @@ __global__ void __launch_bounds__(1024) k_step_scan_layout(Grid G, const int* cn
 // five scans in one, the lists' lengths in shared memory for the receivers'
 // walks (kListCap lists; in global memory beyond), and the counters' bases
 // written where a list's first slot is found.
-constexpr int kListCap = 256 * kMaxNeighbors;
 
 __device__ __forceinline__ void step_layout_body(const Grid& G, const int* pre, int stride,
                                                  const StepTables& T) {
@@ -2013,31 +2085,27 @@ __device__ __forceinline__ void ghost_from_stage_unwrapped(const Arrays& A, cons
 // The plan build's scatter (same outputs as k_halo_scatter, one tile per
 // block) with the tile's records brought into shared memory by bulk copies
 // (every array but the forces, which a ghost does not carry) while the block
-// ranks the tile's hits from the masks.  The images are then written list by
-// list from shared memory, consecutive threads on consecutive ghost slots:
-// the records cross HBM once, as whole tiles, instead of as one 32-byte
-// sector per array and image.  A tile with more images than the staging
-// list holds writes them from HBM reads during the ranking, as k_halo_scatter
-// does.
+// ranks the tile's hits from its bits (index_move: every particle "stays" at
+// its own index).  The images are then written list by list from shared
+// memory, consecutive threads on consecutive ghost slots: the records cross
+// HBM once, as whole tiles, instead of as one 32-byte sector per array and
+// image.  1M particles with 557,000 ghosts of 140 B: 78 us ranking from masks,
+// 53 from the bits.
 __global__ void __launch_bounds__(NT, 4) k_halo_scatter_staged(
-    Grid G, Arrays A, long long owned_off, long long ghost_off, const int4* __restrict__ tiles,
-    const int* ntiles, const unsigned* __restrict__ mask, const int* pre, int stride,
-    const int* cbase, int* ghost_owner, int* ghost_entry, int* bowner, int* boff, int* bslot,
-    int* bfirst) {
+    Grid G, Arrays A, long long owned_off, long long ghost_off, const unsigned* __restrict__ bits,
+    const int* pre, int stride, const int* cbase, MoveOutputs O) {
     pdl_begin();
     extern __shared__ __align__(16) unsigned char s_rec[];
     __shared__ __align__(8) unsigned long long s_bar;
     __shared__ int s_seg[kStagedArrays];
-    __shared__ int s_cnt[NW][32];
-    __shared__ int s_base[32];
-    __shared__ int s_off[kMaxNeighbors + 1];
-    __shared__ unsigned short s_own[kStageCap];
-    const int g = G.tile_first + blockIdx.x;
-    if (g >= tile_limit(G, ntiles) || (*G.status & kStatusGhostOverflow)) return;
-    const int4 td = tiles[g];
-    const int s = td.x, begin = td.y, end = td.z;
+    __shared__ MoveIndex S;
+    const int g = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wbegin = begin + warp * 32 * ITEMS;
+    const int4 td = G.tiles[g];   // (a row for every block of the launch)
+    const unsigned word = lane < ITEMS * kGroupWords
+        ? ro(bits + static_cast<long long>(g) * kTileWords + warp * ITEMS * kGroupWords + lane) : 0u;
+    if (g >= G.tile_start[G.P] || (*G.status & kStatusGhostOverflow)) return;
+    const int s = td.x, begin = td.y, end = td.z;
     const unsigned bar = smem_u32(&s_bar);
     if (warp == 0) {
         if (lane == 0) {
@@ -2047,88 +2115,10 @@ __global__ void __launch_bounds__(NT, 4) k_halo_scatter_staged(
         __syncwarp();
         stage_issue(A, owned_off, begin, end, s_rec, bar, s_seg, lane, 0, 13 + A.f.count, true);
     }
-    const int nn = G.nn[s];
-    const unsigned lt = lanemask_lt();
-    unsigned m[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int i = wbegin + j * 32 + lane;
-        m[j] = i < end ? mask[i] : 0u;
-    }
-    int acc = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) count_group(m[j], nn, lane, acc);
-    s_cnt[warp][lane] = acc;
-    if (threadIdx.x < kHaloCounters) {
-        const int k = threadIdx.x;
-        s_base[k] = cbase[s * kHaloCounters + k] + pre[k * stride + g] - pre[k * stride + td.w];
-    }
-    __syncthreads();
-    if (warp == 0) {
-        int tot = 0;
-        if (lane < nn)
-            for (int w = 0; w < NW; ++w) tot += s_cnt[w][lane];
-        const int incl = warp_inclusive_sum(tot);
-        if (lane < nn) s_off[lane] = incl - tot;
-        if (lane == 31) s_off[nn] = incl;
-    }
-    __syncthreads();
-    const int Q = s_off[nn];
-    const bool staged = Q <= kStageCap;
-    int run = 0, lrun = 0;
-    if (lane < kHaloCounters) {
-        run = s_base[lane];
-        if (lane < nn) lrun = s_off[lane];
-        for (int w = 0; w < warp; ++w) {
-            run += s_cnt[w][lane];
-            lrun += s_cnt[w][lane];
-        }
-    }
-    const double* shift = G.shift + static_cast<long long>(s) * kMaxNeighbors * 3;
-#pragma unroll 1
-    for (int j = 0; j < ITEMS; ++j) {
-        const unsigned mj = m[j];
-        const unsigned any = __ballot_sync(0xffffffffu, mj != 0);
-        if (!any) continue;
-        const int i = wbegin + j * 32 + lane;
-        const int b = __shfl_sync(0xffffffffu, run, kBoundaryCounter) + __popc(any & lt);
-        const int pm = __popc(mj);
-        const int incl = warp_inclusive_sum(pm);
-        const int img = __shfl_sync(0xffffffffu, run, kImageCounter) + incl - pm;
-        if (mj) {
-            bowner[b] = i;
-            boff[b] = img;
-        }
-        int k = 0;
-        const unsigned used = __reduce_or_sync(0xffffffffu, mj);
-        for (unsigned rest = used; rest; rest &= rest - 1) {
-            const int n = __ffs(rest) - 1;
-            const unsigned hit = __ballot_sync(0xffffffffu, (mj >> n) & 1u);
-            const int list_base = __shfl_sync(0xffffffffu, run, n);
-            const int stage_base = __shfl_sync(0xffffffffu, lrun, n);
-            if ((mj >> n) & 1u) {
-                const int rank = __popc(hit & lt);
-                const int slot = list_base + rank;
-                bslot[img + k] = slot;
-                if (k == 0) bfirst[b] = slot;
-                ++k;
-                if (staged) {
-                    s_own[stage_base + rank] = static_cast<unsigned short>(i - begin);
-                } else {
-                    write_ghost(A, owned_off + i, ghost_off + slot, shift + 3 * n);
-                    ghost_owner[slot] = i;
-                    ghost_entry[slot] = s * kMaxNeighbors + n;
-                }
-            }
-            if (lane == n) {
-                run += __popc(hit);
-                lrun += __popc(hit);
-            }
-        }
-        const int group_images = __shfl_sync(0xffffffffu, incl, 31);
-        if (lane == kBoundaryCounter) run += __popc(any);
-        if (lane == kImageCounter) run += group_images;
-    }
+    int base = lane == kStepStay ? begin : 0;
+    if (warp == 0 && lane < kHaloCounters)
+        base = cbase[s * kHaloCounters + lane] + pre[lane * stride + g] - pre[lane * stride + td.w];
+    const MoveTile t = index_move(G, s, word, base, true, 1, S, O);
     // the records must have landed (and every warp's staging list be
     // visible) before the images are written from shared memory
     const bool lost = !bulk_wait(bar);
@@ -2137,25 +2127,16 @@ __global__ void __launch_bounds__(NT, 4) k_halo_scatter_staged(
         if (threadIdx.x == 0) atomicOr(G.status, kStatusCopyTimeout);
         return;
     }
-    if (!staged) return;
     int sg[13];
 #pragma unroll
     for (int a = 0; a < 13; ++a) sg[a] = s_seg[a];
     const int* fseg = s_seg + 13;
-    for (int q = threadIdx.x; q < Q; q += NT) {
-        int lo = 0, hi = nn;   // largest n with s_off[n] <= q
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (s_off[mid] <= q) lo = mid;
-            else hi = mid;
-        }
-        const int n = lo;
-        const int slot = s_base[n] + (q - s_off[n]);
-        const int l = s_own[q];
+    const double* shift = G.shift + static_cast<long long>(s) * kMaxNeighbors * 3;
+    each_image(t, S, [&](int n, int slot, int l) {
         ghost_from_stage_unwrapped(A, s_rec, sg, fseg, l, ghost_off + slot, shift + 3 * n);
-        ghost_owner[slot] = begin + l;
-        ghost_entry[slot] = s * kMaxNeighbors + n;
-    }
+        O.ghost_owner[slot] = begin + l;
+        O.ghost_entry[slot] = s * kMaxNeighbors + n;
+    });
 }
 
 // First boundary owner of every tile of the current layout (tile_b0[g]; the
@@ -3848,30 +3829,33 @@ constexpr int kForceStageBytes = 3 * (TILE * 8 + 32);
 
 void launch_halo_build(const Grid& G, const Arrays& A, long long owned_off, long long ghost_off,
                        const Scratch& S, cudaStream_t s, const PlainLaunch* plain) {
-    per_subdomain(G, plain, [&](const Grid& Gs, int grid) {
-        pdl_launch(k_halo_classify, grid, NT, 0, s, Gs, G.tiles, G.tile_start + G.P, A.d[0] + owned_off,
-                                            A.d[1] + owned_off, A.d[2] + owned_off, S.mask,
-                                            S.cnt, S.stride);
-    });
-    if (S.marks) S.marks->mark(s, "halo_classify");
-    pdl_launch(k_scan_counters, kHaloCounters, 1024, 0, s, S.cnt, S.pre, S.stride, G.tile_start + G.P);
-    if (S.marks) S.marks->mark(s, "halo_scan");
-    pdl_launch(k_halo_layout, 1, 1024, 0, s, G, S.pre, S.stride, S.list_len, S.send_base, S.list_flat,
-               S.g, S.gbase, S.boff, S.halo_info, S.cbase);
-    if (S.marks) S.marks->mark(s, "halo_layout");
     // the tile's records staged in shared memory (all but the forces) when
-    // they fit; plain launches keep the per-image reads
+    // they fit, ranked from bits; plain launches and wider records keep the
+    // masks and the per-image reads
     const int stage = staged_bytes(A) - kForceStageBytes;
-    if (!plain && stage <= kStagedMaxBytes) {
+    const bool staged = !plain && stage <= kStagedMaxBytes;
+    const double *x = A.d[0] + owned_off, *y = A.d[1] + owned_off, *z = A.d[2] + owned_off;
+    if (staged)
+        pdl_launch(k_halo_bits, G.max_tiles, kBitsThreads, 0, s, G, x, y, z, S.cnt, S.stride, S.bits);
+    else
+        per_subdomain(G, plain, [&](const Grid& Gs, int grid) {
+            pdl_launch(k_halo_classify, grid, NT, 0, s, Gs, G.tiles, G.tile_start + G.P, x, y, z, S.mask,
+                       S.cnt, S.stride);
+        });
+    if (S.marks) S.marks->mark(s, "halo_classify");
+    pdl_launch(k_halo_scan_layout, kHaloCounters, 1024, 0, s, G, S.cnt, S.pre, S.stride, S.list_len,
+               S.send_base, S.list_flat, S.g, S.gbase, S.boff, S.halo_info, S.cbase, S.ticket);
+    if (S.marks) S.marks->mark(s, "halo_layout");
+    if (staged) {
         static bool attribute_set = false;   // once per process (one device per process)
         if (!attribute_set) {
             cudaFuncSetAttribute(k_halo_scatter_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kStagedMaxBytes);
             attribute_set = true;
         }
+        const MoveOutputs O{S.ghost_owner, S.ghost_entry, S.bowner, S.boff, S.bslot, S.bfirst};
         pdl_launch(k_halo_scatter_staged, G.max_tiles, NT, static_cast<std::size_t>(stage), s, G, A,
-                   owned_off, ghost_off, G.tiles, G.tile_start + G.P, S.mask, S.pre, S.stride,
-                   S.cbase, S.ghost_owner, S.ghost_entry, S.bowner, S.boff, S.bslot, S.bfirst);
+                   owned_off, ghost_off, S.bits, S.pre, S.stride, S.cbase, O);
     } else {
         per_subdomain(G, plain, [&](const Grid& Gs, int grid) {
             pdl_launch(k_halo_scatter, grid, NT, 0, s, Gs, A, owned_off, ghost_off, G.tiles,
