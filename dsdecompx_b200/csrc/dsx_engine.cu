@@ -459,6 +459,8 @@ struct dsx_grid {
     bool ghosts_valid = false;
     std::vector<long long> last_ghosts;
     unsigned* pinned_status = nullptr;   // [4]: status, G, B, pad
+    unsigned* pinned_report = nullptr;   // the host's image of the block that starts at `status`
+    std::size_t report_g = 0, report_mig = 0, report_flags = 0;   // where its parts start (words)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     dsx::Marks marks;
     dsx_step_callback graph_callback = nullptr;
@@ -502,6 +504,7 @@ struct dsx_grid {
         for (void* p : scratch_owned) cudaFree(p);
         for (void* p : fixed_owned) cudaFree(p);
         if (pinned_status) cudaFreeHost(pinned_status);
+        if (pinned_report) cudaFreeHost(pinned_report);
     }
 
     // Split-phase halo as two captured graph segments: segment 1 is the
@@ -752,10 +755,18 @@ struct dsx_grid {
         }
         const int tiles_cap = static_cast<int>((ncap + dsx::kTile - 1) / dsx::kTile) + P;
         for (auto& t : layout_tiles) t = device_alloc<int4>(fixed_owned, tiles_cap);
-        // the status word, then the plan's totals {G, B} (S.halo_info, four
-        // words): one copy brings the status and the totals to the host
-        status = device_alloc<unsigned>(fixed_owned, 8);
-        cuda_check(cudaMemset(status, 0, 8 * sizeof(unsigned)), "memset");
+        // What calls report, in one block with a pinned image on the host: the
+        // status word and the plan's totals {G, B} (S.halo_info, four words),
+        // the ghosts per receiver, the migration results, and the
+        // out-of-domain flags.  A call's report is one copy and one wait.
+        report_g = 8;
+        report_mig = report_g + (static_cast<std::size_t>(P) + 2) / 2 * 2;
+        report_flags = report_mig + static_cast<std::size_t>(P) * 12;
+        const std::size_t report_words = report_flags + static_cast<std::size_t>(P);
+        status = device_alloc<unsigned>(fixed_owned, report_words);
+        cuda_check(cudaMemset(status, 0, report_words * sizeof(unsigned)), "memset");
+        cuda_check(cudaMallocHost(reinterpret_cast<void**>(&pinned_report), report_words * sizeof(unsigned)),
+                   "cudaMallocHost");
         call_counter = device_alloc<long long>(fixed_owned, 1);
         cuda_check(cudaMemset(call_counter, 0, sizeof(long long)), "memset");
         rebalance_result = device_alloc<double>(fixed_owned, 6);
@@ -790,7 +801,7 @@ struct dsx_grid {
         S.emig_hist = device_alloc<int>(fixed_owned, static_cast<std::size_t>(S.max_chunks) * P);
         S.emig_info = device_alloc<int>(fixed_owned, 4);
         cuda_check(cudaMemset(S.emig_info, 0, 4 * sizeof(int)), "memset");
-        S.mig_results = device_alloc<long long>(fixed_owned, static_cast<std::size_t>(P) * 6);
+        S.mig_results = reinterpret_cast<long long*>(status + report_mig);
         // halo masks per particle (per-call build, immigrants); bits and
         // destinations per tile slot (batched step)
         const std::size_t slots = static_cast<std::size_t>(max_tiles) * dsx::kTile;
@@ -798,13 +809,12 @@ struct dsx_grid {
         S.bits = device_alloc<unsigned>(fixed_owned, static_cast<std::size_t>(max_tiles) * dsx::kTileBits);
         S.dest16 = device_alloc<unsigned short>(fixed_owned, slots);
         S.tile_bases = device_alloc<int>(fixed_owned, static_cast<std::size_t>(max_tiles) * 32);
-        S.out_flags = device_alloc<int>(fixed_owned, P);
+        S.out_flags = reinterpret_cast<int*>(status + report_flags);
         S.list_len = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * E);
         S.send_base = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * E);
         S.list_flat = device_alloc<int>(fixed_owned, static_cast<std::size_t>(P) * E);
-        S.g = device_alloc<int>(fixed_owned, P + 1);
+        S.g = reinterpret_cast<int*>(status + report_g);
         S.gbase = device_alloc<int>(fixed_owned, P + 1);
-        cuda_check(cudaMemset(S.g, 0, sizeof(int) * (P + 1)), "memset");
         cuda_check(cudaMemset(S.gbase, 0, sizeof(int) * (P + 1)), "memset");
         S.bowner = device_alloc<int>(fixed_owned, ncap);
         S.boff = device_alloc<int>(fixed_owned, ncap + 1);
@@ -940,6 +950,14 @@ struct dsx_grid {
         return pinned_status[0];
     }
 
+    // Words [first, last) of the report block to its host image (synchronizes).
+    const unsigned* read_report(std::size_t first, std::size_t last, cudaStream_t stream) {
+        cuda_check(cudaMemcpyAsync(pinned_report + first, status + first, (last - first) * sizeof(unsigned),
+                                   cudaMemcpyDeviceToHost, stream), "read report");
+        cuda_check(cudaStreamSynchronize(stream), "synchronize");
+        return pinned_report + first;
+    }
+
     void clear_status(cudaStream_t stream) {
         cuda_check(cudaMemsetAsync(status, 0, sizeof(unsigned), stream), "clear status");
     }
@@ -979,15 +997,27 @@ struct dsx_grid {
             G.need = d_need_empty;
             dsx::launch_step_classify(G, A, owned_off(), S, stream);
             dsx::launch_step_layout(G, S, stream, desc.policy != DSX_DYNAMIC);
-            dsx::launch_step_bases(G, S, stream);
-            dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);
-            dsx::launch_step_finish(G, G, A, owned_off(), next_off(), ghost_off(), S, stream, false);
+            // a call that waits for its results places the emigrants beside
+            // the move, as the step does (without a wait the stream's next
+            // kernel could have a programmatic edge to the move alone)
+            if (results) {
+                const dsx::Branch branch{emigrant_stream, emigrant_fork, emigrant_join};
+                cuda_check(dsx::fork_branch(branch, stream), "fork");
+                dsx::launch_step_finish(G, G, A, owned_off(), next_off(), ghost_off(), S, branch.stream, false);
+                dsx::launch_step_bases(G, S, stream);
+                dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);
+                cuda_check(dsx::join_branch(branch, stream), "join");
+            } else {
+                dsx::launch_step_bases(G, S, stream);
+                dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);
+                dsx::launch_step_finish(G, G, A, owned_off(), next_off(), ghost_off(), S, stream, false);
+            }
         }
         commit_migrate();
         if (results) {
-            cuda_check(cudaMemcpyAsync(results, S.mig_results, sizeof(long long) * 6 * P,
-                                       cudaMemcpyDeviceToHost, stream), "read migration results");
-            const unsigned st = read_status(stream);
+            const unsigned* report = read_report(0, report_flags, stream);
+            std::memcpy(results, report + report_mig, sizeof(long long) * 6 * P);
+            const unsigned st = report[0];
             if (st & dsx::kStatusMigrationMismatch) fail(DSX_E_RUNTIME, "migration count mismatch");
             if (st & dsx::kStatusCutsInvalid)
                 fail(DSX_E_INVALID, "dynamic cuts must be strictly increasing and span the domain");
@@ -1000,11 +1030,12 @@ struct dsx_grid {
         for (;;) {
             clear_status(stream);
             enqueue_halo_build(stream, plain_layout(stream));
-            const unsigned st = read_status(stream);
-            if (st & dsx::kStatusCopyTimeout)
+            // the ghosts per receiver come with the status, for report_halo
+            const unsigned* report = read_report(0, report_mig, stream);
+            if (report[0] & dsx::kStatusCopyTimeout)
                 fail(DSX_E_RUNTIME, "a bulk copy of particle records did not complete within 1 s");
-            if (!(st & dsx::kStatusGhostOverflow)) break;
-            grow_ghosts(static_cast<long long>(static_cast<int>(pinned_status[1])), stream);
+            if (!(report[0] & dsx::kStatusGhostOverflow)) break;
+            grow_ghosts(static_cast<long long>(static_cast<int>(report[1])), stream);
         }
         plan_valid = true;
         ghosts_valid = true;
@@ -1015,7 +1046,7 @@ struct dsx_grid {
         not_pending("exchange_halo");
         sharded_ghosts = false;
         if (rebuild) plan_valid = false;
-        bool reused = false;
+        bool reused = false, built = false;
         if (P == 1) {
             // one rank owns the whole periodic box: no ghosts (dsDecompX src/halo.cpp:325-350)
             plan_valid = false;
@@ -1025,6 +1056,7 @@ struct dsx_grid {
             reused = true;
         } else if (results) {
             build_checked(stream);
+            built = true;
         } else {
             clear_status(stream);
             enqueue_halo_build(stream);
@@ -1032,16 +1064,19 @@ struct dsx_grid {
             plan_valid = true;
             ghosts_valid = true;
         }
-        report_halo(rebuild, reused, stream, results);
+        report_halo(rebuild, reused, stream, results, built);
     }
 
+    // (counts_read: the report block's image already holds the ghost counts)
     // Per subdomain {ghosts, layout changed, storage reallocated, plan reused}.
-    void report_halo(bool rebuild, bool reused, cudaStream_t stream, long long* results) {
+    void report_halo(bool rebuild, bool reused, cudaStream_t stream, long long* results,
+                     bool counts_read = false) {
         if (results) {
-            std::vector<int> g(static_cast<std::size_t>(P), 0);
-            if (ghosts_valid) g = read_ints(S.g, P, stream);
+            if (ghosts_valid && !counts_read)
+                read_report(report_g, report_g + static_cast<std::size_t>(P), stream);
+            const int* g = reinterpret_cast<const int*>(pinned_report + report_g);
             for (int s = 0; s < P; ++s) {
-                const long long now = ghosts_valid ? g[static_cast<std::size_t>(s)] : 0;
+                const long long now = ghosts_valid ? g[s] : 0;
                 long long* o = results + 4 * s;
                 o[0] = now;
                 o[1] = (rebuild || now != last_ghosts[static_cast<std::size_t>(s)] || (now != 0 && !reused)) ? 1 : 0;
@@ -2679,10 +2714,11 @@ int dsx_grid_out_of_domain(dsx_grid* grid, int* flags, int* any, void* stream) {
         const long long o = grid->owned_off();
         dsx::launch_out_of_domain(grid->params(), grid->A.d[0] + o, grid->A.d[1] + o,
                                   grid->A.d[2] + o, grid->S.out_flags, s);
-        std::vector<int> f = grid->read_ints(grid->S.out_flags, grid->P, s);
+        const int* f = reinterpret_cast<const int*>(
+            grid->read_report(grid->report_flags, grid->report_flags + static_cast<std::size_t>(grid->P), s));
         int hit = 0;
-        for (int v : f) hit |= v;
-        if (flags) std::copy(f.begin(), f.end(), flags);
+        for (int r = 0; r < grid->P; ++r) hit |= f[r];
+        if (flags) std::copy(f, f + grid->P, flags);
         if (any) *any = hit;
     });
 }
