@@ -87,7 +87,7 @@ struct Scratch {
                                   // (the CSR), 2 tile by tile with the owners staged (when the
                                   // stage fits), 3 ghost by ghost, sender by sender and list by
                                   // list where the copied arrays exceed the L2, else as 0
-    int reverse_per_sm = 0;       // CTAs per SM of the reverse sum; 0: one wave of the default shape
+    int reverse_per_sm = 0;       // CTAs per SM of the reverse sum; 0: up to 32, one owner per thread
 };
 
 void launch_layout(const Grid& G, const int* n, int* obase, int* tile_start, int4* tiles,

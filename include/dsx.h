@@ -344,8 +344,8 @@ int dsx_grid_autotune(dsx_grid* grid, void* stream, dsx_tune_report* report);
  * choose them; for re-using a tuning, and for tests that force each kind):
  * classify_threads 64, 128 or 256; move_kind as dsx_tune_report.move_staged
  * (a kind that does not fit the record's shared-memory budget falls back to
- * staged passes or direct reads); reverse_ctas_per_sm 0 (two waves of the
- * grid's SMs) or 1..32; classify_combine as dsx_tune_report.classify_combine.
+ * staged passes or direct reads); reverse_ctas_per_sm 0 (up to 32, one owner
+ * per thread where that is fewer) or 1..32; classify_combine as dsx_tune_report.classify_combine.
  * Results are identical for every setting. */
 int dsx_grid_set_tuning(dsx_grid* grid, int classify_threads, int move_kind,
                         int reverse_ctas_per_sm, int classify_combine);
