@@ -160,12 +160,12 @@ def algorithmic_bytes(S, N, E, G, B):
         "mig_classify": 24 * N,                               # positions
         "mig_move": 24 * N + (S - 24) * R + S * R + 8 * E,    # read all, write retained, list emigrants
         "emig_place": E * (8 + 2 * S),
-        "halo_classify": 24 * N + 4 * N,                      # positions in, mask out
-        "halo_scatter": 4 * N + S * B + (S + 12) * G + 8 * B,  # masks, owners, ghosts + maps
+        "halo_classify": 24 * N + N,                          # positions in, bits out
+        "halo_scatter": N + S * B + (S + 12) * G + 8 * B,  # masks, owners, ghosts + maps
         "reverse_sum": 8 * B + 4 * G + 24 * G + 48 * B,       # CSR, ghost forces, owner RMW
         # fused step (migrate + plan build in one pipeline)
-        "step_classify": 24 * N + 6 * N,                      # positions in; destination + mask out
-        "step_move": 6 * N + S * R + S * R + 8 * E + (S + 12) * G + 8 * B,
+        "step_classify": 24 * N + N,                          # positions in, bits out
+        "step_move": N + S * R + S * R + 8 * E + (S + 12) * G + 8 * B,
         "immigrant_halo": E * (24 + 4),
     }
 
