@@ -3391,13 +3391,14 @@ __device__ __forceinline__ void stage_cuts(const Grid& G, double* s_cuts) {
 // is the count of those the position is not below -- what upper_bound gives on
 // strictly increasing cuts, clamped at both ends; a NaN, below no cut, ends
 // in the last cell as there.  One test per position decides whether any axis
-// needs the wrap's arithmetic.  Two positions a thread, the next two loaded
+// needs the wrap's arithmetic (doing it always, without the test, costs the
+// positions inside more than it saves the others: 70 -> 100 us, 106 -> 99).  Two positions a thread, the next two loaded
 // before these are searched.
 //
 // With no table and no loop a position takes some 45 instructions against 200
 // for the binned search below (which is bound by them): 16M positions, a
-// quarter of them outside the box, 4x4x4 175 -> 108 us, 8x8x4 177 -> 130 us;
-// 5M 57 -> 37 us.
+// quarter of them outside the box, 4x4x4 175 -> 106 us, 8x8x4 177 -> 125 us;
+// 5M 57 -> 36 us; all inside, 4x4x4, 118 -> 70 us (the copy rate).
 template <int MAXD, bool WIDE>
 __global__ void __launch_bounds__(NT, MAXD == 4 ? 4 : 3) k_owner_rank_few(Grid G, const double* __restrict__ x,
                                                        const double* __restrict__ y,
@@ -3422,8 +3423,23 @@ __global__ void __launch_bounds__(NT, MAXD == 4 ? 4 : 3) k_owner_rank_few(Grid G
 #pragma unroll
         for (int a = 0; a < 3; ++a) plain = plain && lo[a] <= v[a] && v[a] < hi[a];
         if (!plain) {
+            // one box to either side (the cases and the reasons of
+            // wrap_axis): one add of a selected value, no division
+            bool near = true;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) v[a] = wrap_if(G, a, v[a]);
+            for (int a = 0; a < 3; ++a) {
+                if (!G.periodic[a]) continue;
+                const double E = G.extent[a], t = __dsub_rn(v[a], G.lower[a]);
+                const double by = t < 0.0 ? E : t >= E ? -E : 0.0;
+                near = near && t < __dadd_rn(E, E) && t >= -E &&
+                       (t >= 0.0 || t <= __dmul_rn(E, -0x1p-500));
+                v[a] = __dadd_rn(__dadd_rn(t, by), G.lower[a]);
+            }
+            if (!near) {
+                v[0] = wrap_if(G, 0, px);
+                v[1] = wrap_if(G, 1, py);
+                v[2] = wrap_if(G, 2, pz);
+            }
         }
         int r = 0;
 #pragma unroll
