@@ -1319,11 +1319,13 @@ struct dsx_grid {
         // exchanges called from it act on these ghosts)
         const bool saved_plan = plan_valid, saved_ghosts = ghosts_valid;
         plan_valid = ghosts_valid = true;
+        // the first library kernel after the join, the callback's or the
+        // reverse sum, waits for both streams in full
+        if (!marks.on) dsx::plain_edge();
         if (cb) cb(user, stream, &v);
         plan_valid = saved_plan;
         ghosts_valid = saved_ghosts;
         marks.mark(stream, "callback");
-        if (!marks.on) dsx::plain_edge();   // the callback may have queued nothing after the join
         enqueue_reverse(stream);
         // the status after the build is the step's (nothing later sets a
         // bit): a step with the build's copy needs no second one

@@ -19,9 +19,17 @@ def check(pair, rng, sigma, steps=2):
         pair.displace(rng, sigma)
         torch.cuda.synchronize()
         if step:      # the batched step, then the calls it stands for
-            assert pair.gpu.step(capture=True, stream=stream) == 0
+            # the callback's first launch is the library's own: it must wait
+            # for the emigrants' branch as well as for the move
+            callback = None
+            if pair.fields:
+                def callback(view, s):
+                    pair.gpu.reverse_exchange([("q", "sum")], stream=s)
+            assert pair.gpu.step(callback, capture=True, stream=stream) == 0
             pair.ref.migrate()
             pair.ref.exchange_halo(rebuild=True)
+            if pair.fields:
+                pair.ref.reverse_exchange([("q", "sum")])
             pair.ref.reverse_halo()
         else:
             assert (pair.gpu.migrate() == pair.ref.migrate()).all()
