@@ -2417,7 +2417,7 @@ __global__ void __launch_bounds__(kImmThreads, 1) k_step_immigrants(
     const int d = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
-    const int base = imm_base[d], expected = imm_total[d];
+    const int base = imm_base[d], expected = imm_total[d], end = base + expected;
     const bool ghosts = !(*G.status & kStatusGhostOverflow);
     if (threadIdx.x < kHaloCounters) s_run[threadIdx.x] = cbase_imm[d * kHaloCounters + threadIdx.x];
     // the immigrants' sources, in the list's order, four entries a thread
@@ -2435,13 +2435,14 @@ __global__ void __launch_bounds__(kImmThreads, 1) k_step_immigrants(
         int total;
         int at = base + n + block_scan_excl<kImmThreads>(m0 + m1 + m2 + m3, total, ws);
         n += total;
-        // past the layout's count only after a mismatch, which is reported
-        if (n <= expected) {
-            if (m0) order[at++] = from.x;
-            if (m1) order[at++] = from.y;
-            if (m2) order[at++] = from.z;
-            if (m3) order[at] = from.w;
-        }
+        // (an entry past the layout's count, after a mismatch, has no slot)
+        if (m0 && at < end) order[at] = from.x;
+        at += m0;
+        if (m1 && at < end) order[at] = from.y;
+        at += m1;
+        if (m2 && at < end) order[at] = from.z;
+        at += m2;
+        if (m3 && at < end) order[at] = from.w;
     }
     if (threadIdx.x == 0 && n != expected) atomicOr(G.status, kStatusMigrationMismatch);
     if (n > expected) n = expected;

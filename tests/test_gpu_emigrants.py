@@ -58,3 +58,17 @@ def test_emigrants_follow_the_oracle(cuda, dims, n, sigma):
         check(pair, rng, sigma)
     finally:
         pair.close()
+
+
+def test_miscounted_emigrants_are_reported(cuda):
+    """tests/cpp/emigrant_sanity.cu: more or fewer leavers than the layout
+    counted raise the status bit, and only the counted slots are written."""
+    import os
+    import subprocess
+
+    import dsdecompx_b200 as dsx
+    exe = os.path.join(os.path.dirname(dsx.library_path()), "emigrant_sanity")
+    assert os.path.exists(exe), "tests/cpp programs are built by __graft_entry__.build()"
+    proc = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert proc.returncode == 0, proc.stdout + proc.stderr
+    assert "emigrant_sanity: ok" in proc.stdout
