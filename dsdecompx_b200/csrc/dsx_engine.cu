@@ -1001,9 +1001,9 @@ struct dsx_grid {
             // the move, as the step does (without a wait the stream's next
             // kernel could have a programmatic edge to the move alone)
             if (results) {
-                const dsx::Branch branch{emigrant_stream, emigrant_fork, emigrant_join};
+                const dsx::Branch branch = emigrant_branch(false);
                 cuda_check(dsx::fork_branch(branch, stream), "fork");
-                dsx::launch_step_finish(G, G, A, owned_off(), next_off(), ghost_off(), S, branch.stream, false);
+                dsx::launch_step_finish(G, G, A, owned_off(), next_off(), ghost_off(), S, branch.stream, false, true);
                 dsx::launch_step_bases(G, S, stream);
                 dsx::launch_step_move(G, A, owned_off(), next_off(), ghost_off(), S, stream);
                 cuda_check(dsx::join_branch(branch, stream), "join");
@@ -1281,6 +1281,11 @@ struct dsx_grid {
         return v;
     }
 
+    // (the fence is a word of the report block that no report holds)
+    dsx::Branch emigrant_branch(bool fence) const {
+        return {emigrant_stream, emigrant_fork, emigrant_join, fence ? status + 7 : nullptr};
+    }
+
     void enqueue_step(dsx_step_callback cb, void* user, cudaStream_t stream, bool build_event = false) {
         marks.count = 0;
         // a Dynamic grid's rebalance opens the step and clears the status;
@@ -1294,7 +1299,7 @@ struct dsx_grid {
             const dsx::Grid Gn = params();
             cur ^= 1;
             // one stream when every kernel is timed by itself
-            const dsx::Branch branch{emigrant_stream, emigrant_fork, emigrant_join};
+            const dsx::Branch branch = emigrant_branch(true);
             cuda_check(dsx::launch_fused_step(G, Gn, A, owned_off(), next_off(), ghost_off(), S, stream,
                                               !dynamic, marks.on ? nullptr : &branch), "launch step");
         }
@@ -1319,9 +1324,6 @@ struct dsx_grid {
         // exchanges called from it act on these ghosts)
         const bool saved_plan = plan_valid, saved_ghosts = ghosts_valid;
         plan_valid = ghosts_valid = true;
-        // the first library kernel after the join, the callback's or the
-        // reverse sum, waits for both streams in full
-        if (!marks.on) dsx::plain_edge();
         if (cb) cb(user, stream, &v);
         plan_valid = saved_plan;
         ghosts_valid = saved_ghosts;

@@ -3724,15 +3724,26 @@ int sm_count() {
 // previous kernel on the stream drains, inside captured graphs too; errors
 // surface through cudaGetLastError like those of triple-chevron launches.
 //
-// The first kernel on a stream after it was joined with another one waits for
-// both in full: a PlainEdge in scope makes the next launch of this thread an
-// ordinary one (the attribute orders a kernel against its stream's own
-// predecessor only).
-thread_local bool t_plain_edge = false;
+// The attribute orders a kernel against its stream's own predecessor only, and
+// capture gives it to every edge into the kernel: the first kernel after a
+// captured stream was joined with another one (more than one node to wait for)
+// is launched without it, whoever made the join and whichever thread launches.
+// (tests/cpp/join_sanity.cpp; on a live stream the library's own join puts a
+// memset between, join_branch.)
+bool joined(cudaStream_t s) {
+    // the legacy stream cannot be captured, nor be asked while others are
+    if (s == nullptr || s == cudaStreamLegacy) return false;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t* from = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    std::size_t n = 0;
+    if (cudaStreamGetCaptureInfo_v3(s, &status, nullptr, nullptr, &from, &edges, &n) != cudaSuccess) return true;
+    return status == cudaStreamCaptureStatusActive && n > 1;
+}
 
 template <class... Params, class... Args>
-void pdl_launch(void (*kernel)(Params...), dim3 grid, int block, std::size_t smem, cudaStream_t s,
-                Args&&... args) {
+void launch(bool overlap, void (*kernel)(Params...), dim3 grid, int block, std::size_t smem, cudaStream_t s,
+            Args&&... args) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -3742,9 +3753,14 @@ void pdl_launch(void (*kernel)(Params...), dim3 grid, int block, std::size_t sme
     config.dynamicSmemBytes = smem;
     config.stream = s;
     config.attrs = attr;
-    config.numAttrs = t_plain_edge ? 0 : 1;
-    t_plain_edge = false;
+    config.numAttrs = overlap ? 1 : 0;
     (void)cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+
+template <class... Params, class... Args>
+void pdl_launch(void (*kernel)(Params...), dim3 grid, int block, std::size_t smem, cudaStream_t s,
+                Args&&... args) {
+    launch(!joined(s), kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 int stream_grid(long long items) {
@@ -3985,8 +4001,9 @@ void launch_step_bases(const Grid& G, const Scratch& S, cudaStream_t s) {
         G, S.pre, S.stride, S.cbase, S.tile_bases);
 }
 
-void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s) {
-    pdl_launch(k_emig_list, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
+void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s,
+                               bool forked) {
+    launch(!forked && !joined(s), k_emig_list, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
         G, S.pre, S.stride, S.bits, S.dest16, S.emig_src, S.emig_dst, imm_in, S.imm_base,
         S.imm_tile_start, S.imm_tiles);
 }
@@ -4066,8 +4083,8 @@ bool few_tiles(const Grid& G) { return G.max_tiles <= kImmigrantTiles; }
 
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
                         long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s,
-                        bool halo) {
-    launch_step_emigrant_list(G, S, S.imm_total, s);
+                        bool halo, bool forked) {
+    launch_step_emigrant_list(G, S, S.imm_total, s, forked);
     if (few_tiles(G)) {
         const MoveOutputs O{S.ghost_owner, S.ghost_entry, S.bowner, S.boff, S.bslot, S.bfirst};
         pdl_launch(k_step_immigrants, G.P, kImmThreads, 0, s, G, A, src_off, dst_off, ghost_off, S.emig_info,
@@ -4098,17 +4115,19 @@ void launch_step_immigrant_halo(const Grid& Gn, const Arrays& A, long long dst_o
 cudaError_t fork_branch(const Branch& b, cudaStream_t s) {
     cudaError_t e = cudaEventRecord(b.fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(b.stream, b.fork, 0);
-    t_plain_edge = true;
     return e;
 }
 
 cudaError_t join_branch(const Branch& b, cudaStream_t s) {
     cudaError_t e = cudaEventRecord(b.join, b.stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b.join, 0);
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (e == cudaSuccess && s != nullptr && s != cudaStreamLegacy) e = cudaStreamIsCapturing(s, &status);
+    // a captured stream's next launch sees that it has two to wait for
+    if (e == cudaSuccess && b.fence && status == cudaStreamCaptureStatusNone)
+        e = cudaMemsetAsync(b.fence, 0, sizeof(unsigned), s);
     return e;
 }
-
-void plain_edge() { t_plain_edge = true; }
 
 cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
                               long long dst_off, long long ghost_off, const Scratch& S,
@@ -4120,7 +4139,7 @@ cudaError_t launch_fused_step(const Grid& G, const Grid& Gn, const Arrays& A, lo
         // the emigrants' and the immigrants' kernels read what the layout
         // left and write slots the move does not: they run beside it
         cudaError_t e = fork_branch(*branch, s);
-        launch_step_finish(G, Gn, A, src_off, dst_off, ghost_off, S, branch->stream);
+        launch_step_finish(G, Gn, A, src_off, dst_off, ghost_off, S, branch->stream, true, true);
         launch_step_bases(G, S, s);
         launch_step_move(G, A, src_off, dst_off, ghost_off, S, s);
         const cudaError_t j = join_branch(*branch, s);

@@ -110,16 +110,17 @@ void launch_halo_build(const Grid& G, const Arrays& A, long long owned_off,
                        const PlainLaunch* plain = nullptr);
 
 // A second stream for kernels that run beside others: fork makes it follow
-// what `s` holds so far, join makes `s` follow it.  The next launch of the
-// calling thread after a fork is ordinary (no programmatic edge); plain_edge()
-// asks the same for the first launch on a joined stream.
+// what `s` holds so far, join makes `s` follow it.  The branch's first launch
+// and the first one after the join are ordinary (no programmatic edge).
+// fence: a device word that nothing reads, written after a join of live
+// streams (null where the host waits for the join).
 struct Branch {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    unsigned* fence = nullptr;
 };
 cudaError_t fork_branch(const Branch& b, cudaStream_t s);
 cudaError_t join_branch(const Branch& b, cudaStream_t s);
-void plain_edge();
 
 // migrate + plan build as one pipeline (the batched step); G: current layout,
 // Gn: the same grid with the next layout current.  branch: where the
@@ -144,14 +145,16 @@ void launch_step_layout(const Grid& G, const Scratch& S, cudaStream_t s, bool fr
 // wait for each other, and the layout reads every copy).
 int immigrant_copies(int P, int max_tiles);
 void launch_step_bases(const Grid& G, const Scratch& S, cudaStream_t s);
-// imm_in: immigrants per subdomain whose ghost images this grid makes
-void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s);
+// imm_in: immigrants per subdomain whose ghost images this grid makes.
+// forked: the first launch of a branch.
+void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s,
+                               bool forked = false);
 void launch_step_move(const Grid& G, const Arrays& A, long long src_off, long long dst_off,
                       long long ghost_off, const Scratch& S, cudaStream_t s);
 // halo false: a migrate alone (its grid's halo table is empty).
 void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long long src_off,
                         long long dst_off, long long ghost_off, const Scratch& S, cudaStream_t s,
-                        bool halo = true);
+                        bool halo = true, bool forked = false);
 // The finish is two launches (few tiles) instead of seven.
 bool few_tiles(const Grid& G);
 // The finish in its two parts: the emigrants' stable multi-split into the

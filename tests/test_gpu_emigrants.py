@@ -60,15 +60,19 @@ def test_emigrants_follow_the_oracle(cuda, dims, n, sigma):
         pair.close()
 
 
-def test_miscounted_emigrants_are_reported(cuda):
+@pytest.mark.parametrize("program", ["emigrant_sanity", "join_sanity"])
+def test_cpp_programs(cuda, program):
     """tests/cpp/emigrant_sanity.cu: more or fewer leavers than the layout
-    counted raise the status bit, and only the counted slots are written."""
+    counted raise the status bit, and only the counted slots are written.
+    tests/cpp/join_sanity.cpp: the first launch after a captured stream was
+    joined with another one (as a step's emigrants' branch is) waits for both
+    in full, whatever was launched in between."""
     import os
     import subprocess
 
     import dsdecompx_b200 as dsx
-    exe = os.path.join(os.path.dirname(dsx.library_path()), "emigrant_sanity")
+    exe = os.path.join(os.path.dirname(dsx.library_path()), program)
     assert os.path.exists(exe), "tests/cpp programs are built by __graft_entry__.build()"
     proc = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert proc.returncode == 0, proc.stdout + proc.stderr
-    assert "emigrant_sanity: ok" in proc.stdout
+    assert f"{program}: ok" in proc.stdout
