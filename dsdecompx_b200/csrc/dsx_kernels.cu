@@ -11,6 +11,8 @@
 // force sums) must round exactly like the reference's.
 #include "dsx_kernels.cuh"
 
+#include <cooperative_groups.h>
+
 #include <cstdio>
 #include <mutex>
 #include <utility>
@@ -2391,49 +2393,82 @@ __global__ void __launch_bounds__(NT) k_emig_list(Grid G, const int* pre, int st
 }
 
 // The emigrants' chain after their list in one launch, for grids of few tiles:
-// one CTA per destination picks its immigrants from the list (in its order),
-// writes their records after the retained ones, and their ghost images and
-// CSR entries after the retained parts of the send lists -- what k_emig_hist,
-// k_emig_colscan, k_emig_place and the immigrants' k_halo_classify,
-// k_scan_counters and k_halo_scatter do in six launches of some 4 us each,
-// whose latency is a small step's time.  Every CTA reads the whole list, so its
-// time grows with the emigrants: 262,000 particles (1,400 leavers) 11 us against
-// 27 for the chain, 500,000 (3,000) 21, beside a move of 26; beyond 1,024 tiles
-// (kImmigrantTiles) the chain, whose time does not grow, is hidden behind the
-// move.
+// a cluster of CTAs per destination picks its immigrants from the list (in its
+// order), writes their records after the retained ones, and their ghost images
+// and CSR entries after the retained parts of the send lists -- what
+// k_emig_hist, k_emig_colscan, k_emig_place and the immigrants'
+// k_halo_classify, k_scan_counters and k_halo_scatter do in six launches of
+// some 4 us each, whose latency is a small step's time.
+//
+// A list of at most kShortList emigrants is left to the first CTA of each
+// cluster (the others return): 262,000 particles (1,400 leavers) 11 us against
+// 27 for the chain, 500,000 (3,000) 21, beside a move of 26.  A longer one (cut
+// planes moved, a restart) is read in as many parts as the cluster has CTAs,
+// once to count and once to write, and its immigrants are dealt to them in
+// runs: the halo counters of a run, counted first, are where the next one
+// starts.  Whole steps (one CTA a destination / a cluster / the chain): 30,000
+// particles in 2x1x1, half of them leaving, 115 / 77 / 79 us; 100,000 in 2x2x2
+// 208 / 138 / 140; 500,000 in 2x1x1, a tenth leaving, 316 / 163 / 147, half of
+// them 1,321 / 454 / 308 (in 2x2x2 761 / 568 / 319).  The chain behind it, with
+// nothing to do for a short list, gave those last cases the chain's time and
+// every other step 3 to 9 us.  Beyond 1,024 tiles (kImmigrantTiles) the chain is
+// hidden behind the move.
 //
 // order: [ncap] scratch, the source of every immigrant by its new slot.
-constexpr int kImmThreads = 512;
-constexpr int kImmWarps = kImmThreads / 32;
+constexpr int kShortList = 4096;
 
-__global__ void __launch_bounds__(kImmThreads, 1) k_step_immigrants(
+template <int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_step_immigrants(
     Grid G, Arrays A, long long src_off, long long dst_off, long long ghost_off, const int* emig_info,
     const int* __restrict__ emig_src, const int* __restrict__ emig_dst, const int* imm_total,
-    const int* imm_base, const int* cbase_imm, int* order, MoveOutputs O) {
+    const int* imm_base, const int* cbase_imm, int* order, int cluster, MoveOutputs O) {
     pdl_begin();
+    constexpr int WARPS = THREADS / 32;
     __shared__ int ws[33];
-    __shared__ int s_cnt[kImmWarps][32];
+    __shared__ int s_cnt[WARPS][32];
     __shared__ int s_run[32];
-    const int d = blockIdx.x;
+    __shared__ int s_found;        // read by the cluster: matches in this CTA's part of the list
+    __shared__ int s_part[32];     // and the halo counters of its immigrants
+    const int d = blockIdx.x / cluster, part = blockIdx.x % cluster;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
+    const int E = emig_info[0];
+    // (the same for every CTA of the cluster, as everything that decides
+    // whether a cluster barrier is reached)
+    const int parts = E <= kShortList ? 1 : cluster;
+    if (part >= parts) return;
     const int base = imm_base[d], expected = imm_total[d], end = base + expected;
     const bool ghosts = !(*G.status & kStatusGhostOverflow);
-    if (threadIdx.x < kHaloCounters) s_run[threadIdx.x] = cbase_imm[d * kHaloCounters + threadIdx.x];
+    // this CTA's part of the list, in whole groups of four
+    const int groups = (E + 3) / 4, per = (groups + parts - 1) / parts;
+    const int begin = min(part * per, groups) * 4, stop = min((part + 1) * per * 4, E);
+    const cooperative_groups::cluster_group peers = cooperative_groups::this_cluster();
+    int n = 0;           // immigrants found so far, in the list's order
+    if (parts > 1) {
+        int mine = 0;
+#pragma unroll 4
+        for (int e = begin + 4 * threadIdx.x; e < stop; e += 4 * THREADS) {
+            const int4 to = ro(reinterpret_cast<const int4*>(emig_dst + e));
+            mine += (to.x == d) + (to.y == d && e + 1 < E) + (to.z == d && e + 2 < E) + (to.w == d && e + 3 < E);
+        }
+        int found;
+        block_scan_excl<THREADS>(mine, found, ws);
+        if (threadIdx.x == 0) s_found = found;
+        peers.sync();
+        for (int r = 0; r < part; ++r) n += *peers.map_shared_rank(&s_found, r);
+    }
     // the immigrants' sources, in the list's order, four entries a thread
-    const int E = emig_info[0];
-    int n = 0;
-    for (int e0 = 0; e0 < E; e0 += 4 * kImmThreads) {
+    for (int e0 = begin; e0 < stop; e0 += 4 * THREADS) {
         const int e = e0 + 4 * threadIdx.x;
         int4 to = make_int4(-1, -1, -1, -1), from = make_int4(0, 0, 0, 0);
-        if (e < E) {   // (the list's storage is whole groups of four)
+        if (e < stop) {   // (the list's storage is whole groups of four)
             to = ro(reinterpret_cast<const int4*>(emig_dst + e));
             from = ro(reinterpret_cast<const int4*>(emig_src + e));
         }
         const bool m0 = to.x == d, m1 = to.y == d && e + 1 < E, m2 = to.z == d && e + 2 < E,
                    m3 = to.w == d && e + 3 < E;
         int total;
-        int at = base + n + block_scan_excl<kImmThreads>(m0 + m1 + m2 + m3, total, ws);
+        int at = base + n + block_scan_excl<THREADS>(m0 + m1 + m2 + m3, total, ws);
         n += total;
         // (an entry past the layout's count, after a mismatch, has no slot)
         if (m0 && at < end) order[at] = from.x;
@@ -2444,15 +2479,57 @@ __global__ void __launch_bounds__(kImmThreads, 1) k_step_immigrants(
         at += m2;
         if (m3 && at < end) order[at] = from.w;
     }
-    if (threadIdx.x == 0 && n != expected) atomicOr(G.status, kStatusMigrationMismatch);
+    if (parts > 1) {
+        peers.sync();   // the order, written by every CTA of the cluster
+        for (int r = part + 1; r < parts; ++r) n += *peers.map_shared_rank(&s_found, r);
+    }
+    if (threadIdx.x == 0 && part == 0 && n != expected) atomicOr(G.status, kStatusMigrationMismatch);
     if (n > expected) n = expected;
     __syncthreads();   // the order, written by every thread
     const TileBounds bounds = halo_bounds(G, d);
     const ListTest list = list_test(G, d, lane);
     const double* shift = G.shift + static_cast<long long>(d) * kMaxNeighbors * 3;
-    for (int r0 = 0; r0 < n; r0 += kImmThreads) {
+    // this CTA's immigrants
+    const int share = (n + parts - 1) / parts;
+    const int head = min(part * share, n), tail = min(head + share, n);
+    if (threadIdx.x < kHaloCounters) s_run[threadIdx.x] = cbase_imm[d * kHaloCounters + threadIdx.x];
+    if (parts > 1 && ghosts) {
+        // their halo counters, for the CTAs after this one
+        int acc = 0, boundary = 0;
+#pragma unroll 2
+        for (int r0 = head; r0 < tail; r0 += THREADS) {
+            const int r = r0 + threadIdx.x;
+            unsigned flags = 0;
+            if (r < tail) {
+                const long long src = src_off + order[base + r];
+                flags = halo_flags(bounds, wrap_if(G, 0, ro(A.d[0] + src)), wrap_if(G, 1, ro(A.d[1] + src)),
+                                   wrap_if(G, 2, ro(A.d[2] + src)));
+            }
+            unsigned w[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) w[k] = __ballot_sync(0xffffffffu, (flags >> k) & 1u);
+            const unsigned members = list_members(list, w);
+            acc += __popc(members);
+            boundary += __popc(__reduce_or_sync(0xffffffffu, members));
+        }
+        const int images = __reduce_add_sync(0xffffffffu, acc);
+        s_cnt[warp][lane] = lane == kBoundaryCounter ? boundary : lane == kImageCounter ? images : acc;
+        __syncthreads();
+        if (warp == 0) {
+            int sum = 0;
+            for (int k = 0; k < WARPS; ++k) sum += s_cnt[k][lane];
+            s_part[lane] = sum;
+        }
+        peers.sync();
+        if (warp == 0 && lane < kHaloCounters)
+            for (int r = 0; r < part; ++r) s_run[lane] += peers.map_shared_rank(s_part, r)[lane];
+    }
+    // the last reads of another CTA's shared memory
+    if (parts > 1) peers.sync();
+    else __syncthreads();
+    for (int r0 = head; r0 < tail; r0 += THREADS) {
         const int r = r0 + threadIdx.x;
-        const bool in = r < n;
+        const bool in = r < tail;
         const int ni = base + r;
         long long src = 0;
         unsigned flags = 0;
@@ -2486,7 +2563,7 @@ __global__ void __launch_bounds__(kImmThreads, 1) k_step_immigrants(
         s_cnt[warp][lane] = lane == kBoundaryCounter ? __popc(any) : lane == kImageCounter ? images : acc;
         __syncthreads();
         int run = lane < kHaloCounters ? s_run[lane] : 0, all = 0;
-        for (int k = 0; k < kImmWarps; ++k) {
+        for (int k = 0; k < WARPS; ++k) {
             const int c = s_cnt[k][lane];
             run += k < warp ? c : 0;
             all += c;
@@ -3742,25 +3819,34 @@ bool joined(cudaStream_t s) {
 }
 
 template <class... Params, class... Args>
-void launch(bool overlap, void (*kernel)(Params...), dim3 grid, int block, std::size_t smem, cudaStream_t s,
-            Args&&... args) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+void launch(bool overlap, int cluster, void (*kernel)(Params...), dim3 grid, int block, std::size_t smem,
+            cudaStream_t s, Args&&... args) {
+    cudaLaunchAttribute attr[2];
+    unsigned attrs = 0;
+    if (overlap) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[attrs].id = cudaLaunchAttributeClusterDimension;
+        attr[attrs].val.clusterDim.x = static_cast<unsigned>(cluster);
+        attr[attrs].val.clusterDim.y = attr[attrs].val.clusterDim.z = 1;
+        ++attrs;
+    }
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = dim3(static_cast<unsigned>(block));
     config.dynamicSmemBytes = smem;
     config.stream = s;
     config.attrs = attr;
-    config.numAttrs = overlap ? 1 : 0;
+    config.numAttrs = attrs;
     (void)cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
 template <class... Params, class... Args>
 void pdl_launch(void (*kernel)(Params...), dim3 grid, int block, std::size_t smem, cudaStream_t s,
                 Args&&... args) {
-    launch(!joined(s), kernel, grid, block, smem, s, std::forward<Args>(args)...);
+    launch(!joined(s), 1, kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 int stream_grid(long long items) {
@@ -4003,7 +4089,7 @@ void launch_step_bases(const Grid& G, const Scratch& S, cudaStream_t s) {
 
 void launch_step_emigrant_list(const Grid& G, const Scratch& S, const int* imm_in, cudaStream_t s,
                                bool forked) {
-    launch(!forked && !joined(s), k_emig_list, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
+    launch(!forked && !joined(s), 1, k_emig_list, stream_grid(static_cast<long long>(G.max_tiles) * 32), NT, 0, s,
         G, S.pre, S.stride, S.bits, S.dest16, S.emig_src, S.emig_dst, imm_in, S.imm_base,
         S.imm_tile_start, S.imm_tiles);
 }
@@ -4075,9 +4161,18 @@ void launch_step_export(const Grid& G, const Scratch& S, int* out, cudaStream_t 
     pdl_launch(k_step_export, 1, 1024, 0, s, G, S.pre, S.stride, out, S.imm_total, S.imm_rep, S.imm_copies);
 }
 
-// Up to this many tiles one CTA per destination handles the emigrants
-// (k_step_immigrants, where the sizes behind the line stand).
+// Up to this many tiles k_step_immigrants handles the emigrants (the sizes
+// behind the line stand there).  A cluster starts when all its CTAs fit at
+// once, beside the move's.  Up to kClusterTiles the move leaves room on most
+// SMs for CTAs of 256 threads and 80 registers (60,000 particles in 3x2x2: 67 us
+// a step as with one CTA, 71 with 512 threads and 104 registers).  Beyond, the
+// move fills the GPU, the larger CTA places more a pass, and many clusters are
+// small ones (200,000 in 2x2x2, 1 / 2 / 8 CTAs: 73.7 / 74.8 / 76.5 us a step; 2x1x1
+// 60.2 with any).  Beyond 32 subdomains, or with fewer particles than a short
+// list has, one CTA a destination is enough (500,000 in 4x4x4, half of them
+// leaving: 256 us, the chain 335).
 constexpr int kImmigrantTiles = 1024;
+constexpr int kClusterTiles = 256;
 
 bool few_tiles(const Grid& G) { return G.max_tiles <= kImmigrantTiles; }
 
@@ -4087,9 +4182,14 @@ void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long lon
     launch_step_emigrant_list(G, S, S.imm_total, s, forked);
     if (few_tiles(G)) {
         const MoveOutputs O{S.ghost_owner, S.ghost_entry, S.bowner, S.boff, S.bslot, S.bfirst};
-        pdl_launch(k_step_immigrants, G.P, kImmThreads, 0, s, G, A, src_off, dst_off, ghost_off, S.emig_info,
-                   S.emig_src, S.emig_dst, S.imm_total, S.imm_base, S.cbase_imm,
-                   reinterpret_cast<int*>(S.mask), O);
+        auto immigrants = [&](auto kernel, int threads, int cluster) {
+            launch(!joined(s), cluster, kernel, G.P * cluster, threads, 0, s, G, A, src_off, dst_off, ghost_off,
+                   S.emig_info, S.emig_src, S.emig_dst, S.imm_total, S.imm_base, S.cbase_imm,
+                   reinterpret_cast<int*>(S.mask), cluster, O);
+        };
+        if (G.ncap <= kShortList || G.P > 32) immigrants(k_step_immigrants<512, 1>, 512, 1);
+        else if (G.max_tiles > kClusterTiles) immigrants(k_step_immigrants<512, 1>, 512, G.P > 4 ? 2 : 8);
+        else immigrants(k_step_immigrants<256, 3>, 256, G.P > 16 ? 4 : 8);
         return;
     }
     launch_step_emigrants(G, A, src_off, dst_off, S, S.imm_total, nullptr, s);

@@ -144,9 +144,9 @@ void run(int leavers, int counted) {
 }  // namespace
 
 int main() {
-    // the count right, one short and one over, inside a pass of the list and
-    // across its passes
-    for (int leavers : {5, 600, 2048, 5001})
+    // the count right, short and over, inside a pass of the list, across its
+    // passes, and across the CTAs of a cluster of either size
+    for (int leavers : {5, 600, 2048, 5001, 20000, 150001})
         for (int off : {0, -1, 1, -4}) run(leavers, leavers + off);
     if (failures) return 1;
     std::printf("emigrant_sanity: ok\n");

@@ -60,6 +60,30 @@ def test_emigrants_follow_the_oracle(cuda, dims, n, sigma):
         pair.close()
 
 
+@pytest.mark.parametrize("dims,n,sigma", [
+    ((2, 2, 2), 30_011, 3.0),        # eight CTAs of 256 threads, several passes each
+    ((3, 3, 2), 20_003, 4.0),        # four
+    ((2, 1, 1), 9_001, 1.8),         # a list that one CTA takes
+    ((2, 1, 1), 11_003, 3.0),        # a list just past it
+    ((2, 1, 1), 140_001, 3.0),       # more than 256 tiles: eight CTAs of 512 threads
+    ((3, 2, 2), 135_007, 3.0),       # two
+], ids=["eight", "four", "one", "just_past", "wide_eight", "wide_two"])
+def test_many_emigrants_share_a_cluster(cuda, dims, n, sigma):
+    rng = np.random.default_rng(n)
+    fields = [("q", "float64", 1), ("v", "float32", 3)] if n < 100_000 else []
+    L = [4.0 * d for d in dims]
+    pair = Pair(int(np.prod(dims)), dims, "manual", (0, 0, 0), L, (True, True, True), 0.5, True,
+                None, fields, particles=n, ghost_capacity=3 * n + 1000)
+    try:
+        data = uniform_particles(rng, n, (0, 0, 0), L, fields)
+        owner = pair.ref.owner_rank(np.stack([data["x"], data["y"], data["z"]], 1))
+        pair.upload(split_by_owner(owner, data, pair.P))
+        check(pair, rng, sigma)
+        assert (pair.gpu.totals()["emigrants"] > 4_096) == (n != 9_001)
+    finally:
+        pair.close()
+
+
 @pytest.mark.parametrize("program", ["emigrant_sanity", "join_sanity"])
 def test_cpp_programs(cuda, program):
     """tests/cpp/emigrant_sanity.cu: more or fewer leavers than the layout
