@@ -66,7 +66,8 @@ struct Grid {
     double upper[3] = {1, 1, 1};
     double extent[3] = {1, 1, 1};   // upper - lower, computed once on the host
     double width = 0.0;             // halo width
-    long long ncap = 0;             // owned half length (= total owned count)
+    long long ncap = 0;             // owned half length
+    long long particles = 0;        // owned particles in the grid
     long long gcap = 0;             // ghost capacity
     int tile = 1024;
     int max_tiles = 1;              // ceil(ncap / tile) + P

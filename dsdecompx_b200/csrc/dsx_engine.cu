@@ -569,6 +569,7 @@ struct dsx_grid {
         }
         G.width = halo_width;
         G.ncap = ncap;
+        G.particles = total;
         G.gcap = gcap;
         G.tile = dsx::kTile;
         G.max_tiles = static_cast<int>((ncap + dsx::kTile - 1) / dsx::kTile) + P;

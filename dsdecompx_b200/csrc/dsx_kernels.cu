@@ -13,6 +13,7 @@
 
 #include <cooperative_groups.h>
 
+#include <cmath>
 #include <cstdio>
 #include <mutex>
 #include <utility>
@@ -4263,22 +4264,47 @@ int refresh_stage_bytes(const Arrays& A, bool positions_only) {
     return bytes;
 }
 
-// Bytes per particle that a full refresh copies.
-int refresh_bytes(const Arrays& A) {
-    int bytes = 48;
-    for (int f = 0; f < A.f.count; ++f) bytes += A.f.bytes[f];
-    return bytes;
+// Whether a walk whose arrays hold boundary particles in `touched` bytes of
+// DRAM atoms goes list by list.
+//
+// Slot order reads a sender's 64-byte atoms again for each of its receivers.
+// Those follow one another along the faster axes; the two along the slowest
+// split axis lie a whole plane of subdomains away, and between them the walk
+// touches about one plane's share of what it reads in all.  While that share,
+// or all of it, stays in the L2 (126 MB), slot order reads every atom once too,
+// and the list walk only adds its searches; so a walk goes list by list where
+// the touched bytes exceed the L2 and a plane's share exceeds a quarter of it
+// (`share`: the forward exchange in slot order holds four times the warps, and
+// its line is higher).
+//
+// Measured, slot order / list by list in us (touched MB, a plane's share).
+// Positions: 3M in 4x4x4 (72, 18) 35.5 / 39.7; 6M in 2x2x2 (141, 70) 114 / 70, in
+// 4x4x4 (141, 35) 99 / 70; 16M in 8x8x4, thin halo (148, 18) 55 / 59, 8% halo
+// (384, 48) 284 / 174.  Full refresh of 104 B: 1.5M in 2x2x2, thin (60, 30) 16.9 /
+// 19.1, 8% halo (153, 76) 78 / 62; 16M in 8x8x4, thin (640, 80) 211 / 186.
+// Forward: 16M of 8 B in 8x8x4 (128, 16) 49 / 71; 6M of 32 B in 8x8x4 (188, 24)
+// 51 / 59, in 4x4x4 (188, 47) 71 / 58; 6M of 56 B in 2x2x2 (336, 168) 226 / 129.
+bool walk_by_list(const Grid& G, double touched, long long share) {
+    int planes = 1;
+    for (int a = 0; a < 3 && planes == 1; ++a) planes = G.dims[a];
+    return touched > (128ll << 20) && touched > static_cast<double>(share) * planes;
 }
+constexpr long long kRefreshShare = 32ll << 20, kForwardShare = 40ll << 20;
 
-// Whether a walk that copies `bytes` of every ghost's owner goes list by list:
-// once the owned arrays it reads exceed half of the L2 (126 MB).  Below that
-// the lists' repeated reads hit the L2 in any order and the list search only
-// costs.  Measured with a cold L2 and 30% boundary particles (slot order /
-// list by list): positions 2M (48 MB) 25.6 / 26.7 us, 4M (96 MB) 44 / 41, 8M
-// 80 / 63; full refresh of 92 B 0.3M (28 MB) 21.5 / 23.5, 1M (92 MB) 49 / 42,
-// 4M 168 / 107; forward of 20 B 2M (40 MB) 25.6 / 25.6, 4M (80 MB) 40 / 36,
-// 8M 75 / 54.
-bool walk_by_list(const Grid& G, int bytes) { return G.ncap * bytes > (64ll << 20); }
+// The bytes of 64-byte atoms that hold a boundary particle, of an array of
+// `bytes` a particle: from the mean cell's boundary layer, so that no count has
+// to come back from the device.
+double touched_bytes(const Grid& G, int bytes) {
+    double inner = 1.0;   // the part of a mean cell that no list takes
+    for (int a = 0; a < 3; ++a) {
+        if (G.dims[a] == 1) continue;
+        const double faces = G.periodic[a] ? 2.0 : 2.0 * (G.dims[a] - 1) / G.dims[a];
+        const double layer = faces * G.width * G.dims[a] / G.extent[a];
+        inner *= layer < 1.0 ? 1.0 - layer : 0.0;
+    }
+    const double in_atom = bytes < 64 ? 64.0 / bytes : 1.0;
+    return static_cast<double>(G.particles) * bytes * (1.0 - std::pow(inner, in_atom));
+}
 
 void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, long long ghost_off,
                          bool positions_only, const Scratch& S, cudaStream_t s, int ctas_per_sm) {
@@ -4324,7 +4350,10 @@ void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, lo
                                                   S.bfirst, S.ghost_entry);
         return;
     }
-    const bool by_list = S.refresh_kind == 3 && walk_by_list(G, positions_only ? 24 : refresh_bytes(A));
+    double touched = (positions_only ? 3 : 6) * touched_bytes(G, 8);
+    if (!positions_only)
+        for (int f = 0; f < A.f.count; ++f) touched += touched_bytes(G, A.f.bytes[f]);
+    const bool by_list = S.refresh_kind == 3 && walk_by_list(G, touched, kRefreshShare);
     auto walk = [&](auto kernel) {
         int rows = 0;
         int grid = by_list ? walk_grid(reinterpret_cast<const void*>(kernel), G.gcap, rows)
@@ -4340,9 +4369,9 @@ void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, lo
 void launch_forward_fields(const Grid& G, const Arrays& A, long long owned_off,
                            long long ghost_off, const FieldOps& F, const Scratch& S,
                            cudaStream_t s) {
-    int bytes = 0;
-    for (int t = 0; t < F.count; ++t) bytes += A.f.bytes[F.index[t]];
-    if (walk_by_list(G, bytes)) {
+    double touched = 0.0;
+    for (int t = 0; t < F.count; ++t) touched += touched_bytes(G, A.f.bytes[F.index[t]]);
+    if (walk_by_list(G, touched, kForwardShare)) {
         int rows = 0;
         const int grid = walk_grid(reinterpret_cast<const void*>(k_forward_by_list), G.gcap, rows);
         pdl_launch(k_forward_by_list, grid, NT, 0, s, A, owned_off, ghost_off, F, G.P * kMaxNeighbors,
