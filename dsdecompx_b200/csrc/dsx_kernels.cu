@@ -2885,7 +2885,6 @@ __global__ void __launch_bounds__(NT, POSITIONS ? 4 : 2) k_halo_refresh(Grid G, 
     const int lists = G.P * kMaxNeighbors;
     const long long warps = static_cast<long long>(gridDim.x) * NW;
     const int rows = fixed_rows ? fixed_rows : walk_height(total, warps);
-    const long long stride = BY_LIST ? 32 : warps * 32;
     for (long long t0 = (static_cast<long long>(blockIdx.x) * NW + (threadIdx.x >> 5)) * 32 *
                         (BY_LIST ? rows : 1);
          t0 < total; t0 += warps * 32 * rows) {
@@ -2893,7 +2892,7 @@ __global__ void __launch_bounds__(NT, POSITIONS ? 4 : 2) k_halo_refresh(Grid G, 
         if constexpr (BY_LIST) {
             walk_rows(list_flat, send_base, lists, static_cast<int>(t0), rows, total, slot, entry);
         } else {
-            slot_rows(t0, stride, rows, total, slot);
+            slot_rows(t0, warps * 32, rows, total, slot);
 #pragma unroll
             for (int u = 0; u < kWalkRows; ++u)
                 entry[u] = slot[u] >= 0 ? ro(ghost_entry + slot[u]) : 0;
@@ -2930,6 +2929,55 @@ __global__ void __launch_bounds__(NT, POSITIONS ? 4 : 2) k_halo_refresh(Grid G, 
                     if (slot[u] >= 0) A.d[3 + a][ghost_off + slot[u]] = v[u][a];
             for (int f = 0; f < A.f.count; ++f)
                 copy_rows<3>(A.f.base[f], A.f.bytes[f], owned_off, ghost_off, own, slot);
+        }
+    }
+}
+
+// The refresh in slot order of positions alone, and of records of few fields:
+// four ghosts a thread, whose positions are in flight together; the rest is
+// copied ghost by ghost.  64 registers hold twice the warps of the rows
+// above, which is worth more than their loads in flight while the arrays are
+// in the L2 (rows / this, us: full refresh of 48 B, 0.5M in 10x10x10 42 / 39, 0.6M
+// in 8x8x4 29.1 / 27.7; positions, 6M in 8x8x4 71.9 / 69.4), and no longer from
+// three fields on (0.6M in 8x8x4, six fields of 48 B, 54 / 57; 3M 133 / 143).
+template <bool POSITIONS>
+__global__ void __launch_bounds__(NT, 4) k_halo_refresh_slots(Grid G, Arrays A, long long owned_off,
+                                                              long long ghost_off, const int* info,
+                                                              const int* __restrict__ ghost_owner,
+                                                              const int* __restrict__ ghost_entry) {
+    pdl_begin();
+    if (*G.status & kStatusGhostOverflow) return;
+    const int total = info[0];
+    constexpr int U = 4;
+    const long long step = static_cast<long long>(gridDim.x) * NT;
+    for (long long s0 = blockIdx.x * static_cast<long long>(NT) + threadIdx.x; s0 < total; s0 += U * step) {
+        int own[U], ent[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long slot = s0 + u * step;
+            own[u] = slot < total ? ro(ghost_owner + slot) : 0;
+            ent[u] = slot < total ? ro(ghost_entry + slot) : 0;
+        }
+        double p[U][3];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (s0 + u * step < total)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) p[u][a] = A.d[a][owned_off + own[u]];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (s0 + u * step >= total) continue;
+            const long long src = owned_off + own[u], gi = ghost_off + s0 + u * step;
+            const double* sh = G.shift + 3ll * ent[u];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) A.d[a][gi] = __dadd_rn(p[u][a], sh[a]);
+#pragma unroll
+            for (int a = 6; a < 9; ++a) A.d[a][gi] = 0.0;
+            if constexpr (!POSITIONS) {
+#pragma unroll
+                for (int a = 3; a < 6; ++a) A.d[a][gi] = A.d[a][src];
+                copy_fields(A.f, src, gi);
+            }
         }
     }
 }
@@ -4289,6 +4337,8 @@ bool walk_by_list(const Grid& G, double touched, long long share) {
     for (int a = 0; a < 3 && planes == 1; ++a) planes = G.dims[a];
     return touched > (128ll << 20) && touched > static_cast<double>(share) * planes;
 }
+// fields from which a refresh in slot order goes row by row (k_halo_refresh_slots)
+constexpr int kRowFields = 3;
 constexpr long long kRefreshShare = 32ll << 20, kForwardShare = 40ll << 20;
 
 // The bytes of 64-byte atoms that hold a boundary particle, of an array of
@@ -4354,6 +4404,15 @@ void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, lo
     if (!positions_only)
         for (int f = 0; f < A.f.count; ++f) touched += touched_bytes(G, A.f.bytes[f]);
     const bool by_list = S.refresh_kind == 3 && walk_by_list(G, touched, kRefreshShare);
+    // in slot order: positions, and records of few fields
+    if (!by_list && (positions_only || A.f.count < kRowFields)) {
+        const auto kernel = positions_only ? k_halo_refresh_slots<true> : k_halo_refresh_slots<false>;
+        int grid = resident_grid(reinterpret_cast<const void*>(kernel), G.gcap);
+        if (ctas_per_sm > 0 && grid > sm_count() * ctas_per_sm) grid = sm_count() * ctas_per_sm;
+        pdl_launch(kernel, grid, NT, 0, s, G, A, owned_off, ghost_off, S.halo_info, S.ghost_owner,
+                   S.ghost_entry);
+        return;
+    }
     auto walk = [&](auto kernel) {
         int rows = 0;
         int grid = by_list ? walk_grid(reinterpret_cast<const void*>(kernel), G.gcap, rows)
@@ -4362,7 +4421,7 @@ void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, lo
         pdl_launch(kernel, grid, NT, 0, s, G, A, owned_off, ghost_off, S.halo_info, S.list_flat,
                    S.send_base, S.ghost_owner, S.ghost_entry, rows);
     };
-    if (positions_only) by_list ? walk(k_halo_refresh<true, true>) : walk(k_halo_refresh<true, false>);
+    if (positions_only) walk(k_halo_refresh<true, true>);
     else by_list ? walk(k_halo_refresh<false, true>) : walk(k_halo_refresh<false, false>);
 }
 

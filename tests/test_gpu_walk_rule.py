@@ -131,7 +131,7 @@ def test_small_reuse_distances_keep_slot_order(cuda, dims, n, halo, fields, call
     grid, _ = make(dims, n, halo, (True, True, True), fields)
     if call == "positions":
         names = kernels(lambda: grid.exchange_halo(positions_only=True, results=False))
-        assert any("k_halo_refresh<true, false>" in k for k in names), names
+        assert any("k_halo_refresh_slots<true>" in k for k in names), names
     else:
         names = kernels(lambda: grid.forward_exchange([f[0] for f in fields]))
         assert any("k_forward_fields" in k for k in names), names
@@ -143,4 +143,28 @@ def test_capacity_does_not_choose_the_walk(cuda):
     grid, _ = make((2, 2, 2), 300_000, 0.05, (True, True, True), FLUID, particles=8_000_000)
     names = kernels(lambda: grid.exchange_halo(results=False))
     assert any("k_halo_refresh<false, false>" in k for k in names), names
+    grid.close()
+
+
+@pytest.mark.parametrize("fields", [[], FLUID[:2], FLUID[:3]], ids=["none", "two", "three"])
+@pytest.mark.parametrize("positions_only", [False, True], ids=["full", "positions"])
+def test_slot_order_by_ghost_and_by_row(cuda, fields, positions_only):
+    """Both forms of the walk in slot order against the walk owner by owner."""
+    import torch
+
+    grid, ghosts = make((3, 2, 2), 40_003, 0.2, (True, False, True), fields)
+    words = ghost_words(grid, ghosts, fields)
+    results = []
+    for kind in ("owners", "ghosts"):
+        grid.set_refresh_kind(kind)
+        for name in ["x", "y", "z", "fx", "fy", "fz"] + ([] if positions_only else
+                                                         ["vx", "vy", "vz"] + [f[0] for f in fields]):
+            words[name].fill_(-1)
+        torch.cuda.synchronize()
+        names = kernels(lambda: grid.exchange_halo(positions_only=positions_only, results=False))
+        results.append({k: w.clone() for k, w in words.items()})
+    by_row = len(fields) >= 3 and not positions_only
+    assert any(("k_halo_refresh<" if by_row else "k_halo_refresh_slots<") in k for k in names), names
+    for k in words:
+        assert torch.equal(results[0][k], results[1][k]), k
     grid.close()
