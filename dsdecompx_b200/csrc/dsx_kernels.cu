@@ -2750,10 +2750,33 @@ __global__ void __launch_bounds__(NT, 3) k_step_move_staged(
 // few).
 constexpr int kWalkRows = 4;
 
+// How a launch splits such a walk.  The grid is made for the ghosts that the
+// storage can hold, the split for those that the plan has: from `window_from`
+// ghosts on in full rows over the whole grid, below that evenly over the
+// warps of its first `resident` CTAs.
+struct WalkShape {
+    int resident;
+    int window_from;
+};
+
+struct Walk {
+    int rows;
+    int step;   // warps
+    __device__ __forceinline__ Walk(int total, const WalkShape& s);
+};
+
 __device__ __forceinline__ int walk_height(int total, long long warps) {
     const long long rows = (total + 32 * warps - 1) / (32 * warps);
     const long long passes = (rows + kWalkRows - 1) / kWalkRows;
     return passes < 1 ? 1 : static_cast<int>((rows + passes - 1) / passes);
+}
+
+// (a CTA that the walk does not take has no rows)
+__device__ __forceinline__ Walk::Walk(int total, const WalkShape& s) {
+    const bool window = total >= s.window_from;
+    const int ctas = window ? gridDim.x : min(static_cast<int>(gridDim.x), s.resident);
+    step = ctas * NW;
+    rows = static_cast<int>(blockIdx.x) >= ctas ? 0 : window ? kWalkRows : walk_height(total, step);
 }
 
 // The largest e in [0, lists) with flat[e] <= t, by a whole warp (32 probes a
@@ -2878,13 +2901,15 @@ __global__ void __launch_bounds__(NT, POSITIONS ? 4 : 2) k_halo_refresh(Grid G, 
                                                      const int* __restrict__ send_base,
                                                      const int* __restrict__ ghost_owner,
                                                      const int* __restrict__ ghost_entry,
-                                                     int fixed_rows) {
+                                                     WalkShape shape) {
     pdl_begin();
     if (*G.status & kStatusGhostOverflow) return;
     const int total = info[0];
     const int lists = G.P * kMaxNeighbors;
-    const long long warps = static_cast<long long>(gridDim.x) * NW;
-    const int rows = fixed_rows ? fixed_rows : walk_height(total, warps);
+    const Walk walk(total, shape);
+    const int rows = walk.rows;
+    if (!rows) return;
+    const long long warps = walk.step;
     for (long long t0 = (static_cast<long long>(blockIdx.x) * NW + (threadIdx.x >> 5)) * 32 *
                         (BY_LIST ? rows : 1);
          t0 < total; t0 += warps * 32 * rows) {
@@ -2949,12 +2974,12 @@ __global__ void __launch_bounds__(NT, 4) k_halo_refresh_slots(Grid G, Arrays A, 
     if (*G.status & kStatusGhostOverflow) return;
     const int total = info[0];
     constexpr int U = 4;
-    const long long step = static_cast<long long>(gridDim.x) * NT;
-    for (long long s0 = blockIdx.x * static_cast<long long>(NT) + threadIdx.x; s0 < total; s0 += U * step) {
+    const int step = gridDim.x * NT;
+    for (int s0 = blockIdx.x * NT + threadIdx.x; s0 < total; s0 += U * step) {
         int own[U], ent[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const long long slot = s0 + u * step;
+            const int slot = s0 + u * step;
             own[u] = slot < total ? ro(ghost_owner + slot) : 0;
             ent[u] = slot < total ? ro(ghost_entry + slot) : 0;
         }
@@ -3087,12 +3112,14 @@ __global__ void __launch_bounds__(NT, 4) k_forward_by_list(Arrays A, long long o
                                                            const int* __restrict__ list_flat,
                                                            const int* __restrict__ send_base,
                                                            const int* __restrict__ ghost_owner,
-                                                           const unsigned* status, int fixed_rows) {
+                                                           const unsigned* status, WalkShape shape) {
     pdl_begin();
     if (*status & kStatusGhostOverflow) return;
     const int total = info[0];
-    const long long warps = static_cast<long long>(gridDim.x) * NW;
-    const int rows = fixed_rows ? fixed_rows : walk_height(total, warps);
+    const Walk walk(total, shape);
+    const int rows = walk.rows;
+    if (!rows) return;
+    const long long warps = walk.step;
     for (long long t0 = (static_cast<long long>(blockIdx.x) * NW + (threadIdx.x >> 5)) * 32 * rows;
          t0 < total; t0 += warps * 32 * rows) {
         int slot[kWalkRows], entry[kWalkRows], own[kWalkRows];
@@ -3948,16 +3975,18 @@ int resident_grid(const void* kernel, long long items) {
     return static_cast<int>(g < 1 ? 1 : g);
 }
 
-// Grid of a walk by list: a window of full rows where that is six resident
-// waves and more; below that the last wave's share of empty CTAs costs more
-// than the window gains, and one resident wave with its rows spread evenly
-// (rows 0) is faster (full refresh of 12 arrays, resident / window: 1M 35 / 41
-// us, 2M 56 / 63, 4M 102 / 102, 8M 187 / 173).
-int walk_grid(const void* kernel, long long ghosts, int& rows) {
-    const long long chunks = (ghosts + kWalkRows - 1) / kWalkRows;
-    const long long blocks = (chunks + NT - 1) / NT;
-    rows = blocks >= 6ll * sm_count() * blocks_per_sm(kernel) ? kWalkRows : 0;
-    return rows ? window_grid(chunks) : resident_grid(kernel, ghosts);
+// Grid of a walk by list: a window of full rows where those are ten CTAs an SM
+// and more (1.5M ghosts; positions of 2.0M ghosts, resident / window: 81 / 74 us,
+// forward of 2.8M 98 / 92); below that the last wave's share of empty CTAs costs
+// more than the window gains, and one resident wave with its rows spread evenly
+// is faster (positions of 0.3M ghosts 22 / 24 us; full refresh of 12 arrays, 1M
+// particles 35 / 41, 2M 56 / 63, 4M 102 / 102, 8M 187 / 173).
+int walk_grid(const void* kernel, long long ghosts, WalkShape& shape) {
+    const long long full = 10ll * sm_count() * NT * kWalkRows;
+    shape.resident = resident_grid(kernel, ghosts);
+    shape.window_from = full < INT_MAX ? static_cast<int>(full) : INT_MAX;
+    const int window = window_grid((ghosts + kWalkRows - 1) / kWalkRows);
+    return ghosts >= full && window > shape.resident ? window : shape.resident;
 }
 
 }  // namespace
@@ -4414,12 +4443,12 @@ void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, lo
         return;
     }
     auto walk = [&](auto kernel) {
-        int rows = 0;
-        int grid = by_list ? walk_grid(reinterpret_cast<const void*>(kernel), G.gcap, rows)
+        WalkShape shape{INT_MAX, INT_MAX};
+        int grid = by_list ? walk_grid(reinterpret_cast<const void*>(kernel), G.gcap, shape)
                            : resident_grid(reinterpret_cast<const void*>(kernel), G.gcap);
         if (ctas_per_sm > 0 && grid > sm_count() * ctas_per_sm) grid = sm_count() * ctas_per_sm;
         pdl_launch(kernel, grid, NT, 0, s, G, A, owned_off, ghost_off, S.halo_info, S.list_flat,
-                   S.send_base, S.ghost_owner, S.ghost_entry, rows);
+                   S.send_base, S.ghost_owner, S.ghost_entry, shape);
     };
     if (positions_only) walk(k_halo_refresh<true, true>);
     else by_list ? walk(k_halo_refresh<false, true>) : walk(k_halo_refresh<false, false>);
@@ -4431,10 +4460,10 @@ void launch_forward_fields(const Grid& G, const Arrays& A, long long owned_off,
     double touched = 0.0;
     for (int t = 0; t < F.count; ++t) touched += touched_bytes(G, A.f.bytes[F.index[t]]);
     if (walk_by_list(G, touched, kForwardShare)) {
-        int rows = 0;
-        const int grid = walk_grid(reinterpret_cast<const void*>(k_forward_by_list), G.gcap, rows);
+        WalkShape shape;
+        const int grid = walk_grid(reinterpret_cast<const void*>(k_forward_by_list), G.gcap, shape);
         pdl_launch(k_forward_by_list, grid, NT, 0, s, A, owned_off, ghost_off, F, G.P * kMaxNeighbors,
-                   S.halo_info, S.list_flat, S.send_base, S.ghost_owner, G.status, rows);
+                   S.halo_info, S.list_flat, S.send_base, S.ghost_owner, G.status, shape);
     } else {
         pdl_launch(k_forward_fields, resident_grid(reinterpret_cast<const void*>(k_forward_fields), G.gcap), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
                                                             S.ghost_owner, G.status);

@@ -120,6 +120,20 @@ def test_list_walk_leaves_what_slot_order_does(cuda, dims, n, halo, periodic, fi
     grid.close()
 
 
+@pytest.mark.parametrize("n,halo,ghost_capacity,fields,positions_only", [
+    (3_000_001, 0.02, 16_000_000, FLUID, False),    # far fewer ghosts than the capacity's split
+    (8_000_003, 0.06, 16_000_000, [], True),
+    (8_000_009, 0.15, 0, [], True),                 # whole rows over the whole grid
+    (2_000_003, 0.28, 40_000_000, FLUID, False),
+], ids=["reserved", "reserved_positions", "window_positions", "window_reserved"])
+def test_list_walk_splits_by_the_plan(cuda, n, halo, ghost_capacity, fields, positions_only):
+    grid, ghosts = make((2, 2, 2), n, halo, (True, True, True), fields, ghost_capacity=ghost_capacity)
+    names = kernels(lambda: grid.exchange_halo(positions_only=positions_only, results=False))
+    assert any(f"k_halo_refresh<{str(positions_only).lower()}, true>" in k for k in names), names
+    check_walks(grid, ghosts, fields, positions_only)
+    grid.close()
+
+
 @pytest.mark.parametrize("dims,n,halo,fields,call", [
     # what slot order touches between two of a sender's receivers fits the L2
     ((8, 8, 4), 4_000_000, 0.05, [], "positions"),
