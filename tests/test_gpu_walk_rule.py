@@ -17,8 +17,9 @@ class Address:
                                          "typestr": "<" + typestr, "version": 3}
 
 
-def make(dims, n, halo, periodic, fields, ghost_capacity=0, particles=0):
-    """A grid of unit cells with n uniform particles and its halo plan."""
+def make(dims, n, halo, periodic, fields, ghost_capacity=0, particles=0, edge=0.0):
+    """A grid of unit cells with n uniform particles (edge: their x that far
+    above a cell's lower face at most) and its halo plan."""
     import torch
 
     import dsdecompx_b200 as dsx
@@ -26,6 +27,8 @@ def make(dims, n, halo, periodic, fields, ghost_capacity=0, particles=0):
     gen = torch.Generator("cuda").manual_seed(n)
     P = dims[0] * dims[1] * dims[2]
     pos = [torch.rand(n, generator=gen, dtype=torch.float64, device="cuda") * d for d in dims]
+    if edge:
+        pos[0] = pos[0].floor() + edge * (pos[0] - pos[0].floor())
     cell = [v.long().clamp(max=d - 1) for v, d in zip(pos, dims)]
     owner = (cell[0] * dims[1] + cell[1]) * dims[2] + cell[2]
     order = torch.sort(owner, stable=True)[1]
@@ -181,4 +184,32 @@ def test_slot_order_by_ghost_and_by_row(cuda, fields, positions_only):
     assert any(("k_halo_refresh<" if by_row else "k_halo_refresh_slots<") in k for k in names), names
     for k in words:
         assert torch.equal(results[0][k], results[1][k]), k
+    grid.close()
+
+
+def test_reverse_sum_of_more_owners_than_expected(cuda):
+    """Every particle on the boundary, where the mean cell has a ninth there."""
+    import torch
+
+    grid, ghosts = make((2, 2, 2), 1_000_003, 0.02, (True, True, True), [], edge=0.015)
+    assert grid.totals()["boundary"] == 1_000_003
+    words = ghost_words(grid, ghosts, [])
+    v = grid.view()
+    owned = [torch.as_tensor(Address(grid, v.base[6 + a] + v.owned_offset * 8, v.particles, "f8"), device="cuda")
+             for a in range(3)]
+    gen = torch.Generator("cuda").manual_seed(3)
+    force = torch.randn(3, ghosts, generator=gen, dtype=torch.float64, device="cuda")
+    results = []
+    for per_sm in (32, 0):
+        grid.set_tuning(reverse_ctas_per_sm=per_sm)
+        for a in range(3):
+            owned[a].fill_(0.5)
+            words["f" + "xyz"[a]].copy_(force[a].view(torch.int32))
+        torch.cuda.synchronize()
+        grid.reverse_halo()
+        torch.cuda.synchronize()
+        results.append([t.clone() for t in owned])
+    for a in range(3):
+        assert not torch.equal(results[0][a], torch.full_like(owned[a], 0.5))
+        assert torch.equal(results[0][a], results[1][a]), a
     grid.close()
