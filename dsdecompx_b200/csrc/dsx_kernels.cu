@@ -3887,6 +3887,8 @@ bool joined(cudaStream_t s) {
     // the legacy stream cannot be captured, nor be asked while others are
     if (s == nullptr || s == cudaStreamLegacy) return false;
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) return true;
+    if (status != cudaStreamCaptureStatusActive) return false;   // (the cheaper question first)
     const cudaGraphNode_t* from = nullptr;
     const cudaGraphEdgeData* edges = nullptr;
     std::size_t n = 0;
