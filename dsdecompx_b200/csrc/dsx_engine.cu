@@ -472,15 +472,13 @@ struct dsx_grid {
     // reverse sum still run.
     unsigned* pinned_build = nullptr;             // [8]: per parity status, G, B, pad
     cudaEvent_t build_done[2] = {nullptr, nullptr};
-    // the build-status copy runs on a branch of the step graph, so the
-    // callback does not wait for it (fork and join events, side stream)
+    // Branches of a step beside its main stream, one after the other: the
+    // emigrants' and immigrants' kernels beside the move, then the copy of the
+    // build status, which the callback does not wait for.  The stream has the
+    // highest priority: the branch's few blocks go in as the move's many
+    // retire, instead of after all of them.
     cudaStream_t side_stream = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
-    // the emigrants' and immigrants' kernels beside the step's move, on a
-    // stream of the highest priority: their few blocks go in as the move's
-    // many retire, instead of after all of them
-    cudaStream_t emigrant_stream = nullptr;
-    cudaEvent_t emigrant_fork = nullptr, emigrant_join = nullptr;
     bool async_inflight = false;                  // a step whose status is unchecked
     int async_parity = 0;
     unsigned async_status = 0;                    // bits of the checked asynchronous steps
@@ -494,16 +492,11 @@ struct dsx_grid {
         if (fork_ev) cudaEventDestroy(fork_ev);
         if (join_ev) cudaEventDestroy(join_ev);
         if (side_stream) cudaStreamDestroy(side_stream);
-        if (emigrant_fork) cudaEventDestroy(emigrant_fork);
-        if (emigrant_join) cudaEventDestroy(emigrant_join);
-        if (emigrant_stream) cudaStreamDestroy(emigrant_stream);
-        if (pinned_build) cudaFreeHost(pinned_build);
         free_shard_buffers();
         for (auto& e : marks.ev) if (e) cudaEventDestroy(e);
         for (void* p : arrays_owned) cudaFree(p);
         for (void* p : scratch_owned) cudaFree(p);
         for (void* p : fixed_owned) cudaFree(p);
-        if (pinned_status) cudaFreeHost(pinned_status);
         if (pinned_report) cudaFreeHost(pinned_report);
     }
 
@@ -636,20 +629,13 @@ struct dsx_grid {
         allocate_fixed();
         allocate_arrays();
         allocate_ghost_scratch();
-        cuda_check(cudaMallocHost(reinterpret_cast<void**>(&pinned_status), 4 * sizeof(unsigned)),
-                   "cudaMallocHost");
-        cuda_check(cudaMallocHost(reinterpret_cast<void**>(&pinned_build), 8 * sizeof(unsigned)),
-                   "cudaMallocHost");
         for (auto& e : build_done)
             cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "create event");
         cuda_check(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming), "create event");
         cuda_check(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming), "create event");
-        cuda_check(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking), "create stream");
         int lowest = 0, highest = 0;
         cuda_check(cudaDeviceGetStreamPriorityRange(&lowest, &highest), "stream priorities");
-        cuda_check(cudaStreamCreateWithPriority(&emigrant_stream, cudaStreamNonBlocking, highest), "create stream");
-        cuda_check(cudaEventCreateWithFlags(&emigrant_fork, cudaEventDisableTiming), "create event");
-        cuda_check(cudaEventCreateWithFlags(&emigrant_join, cudaEventDisableTiming), "create event");
+        cuda_check(cudaStreamCreateWithPriority(&side_stream, cudaStreamNonBlocking, highest), "create stream");
         S.marks = &marks;
         last_ghosts.assign(static_cast<std::size_t>(P), 0);
     }
@@ -719,10 +705,15 @@ struct dsx_grid {
         d_sender_of = device_alloc<int>(fixed_owned, sender_of.size());
         d_shift = device_alloc<double>(fixed_owned, shift.size());
         d_dir = device_alloc<signed char>(fixed_owned, dir.size());
-        d_lut = device_alloc<unsigned>(fixed_owned, lut.size());
-        d_lut_empty = device_alloc<unsigned>(fixed_owned, lut.size());
-        d_need = device_alloc<unsigned char>(fixed_owned, need.size());
-        d_need_empty = device_alloc<unsigned char>(fixed_owned, need.size());
+        // both tables of a list's comparisons, then the empty ones
+        const std::size_t tables = lut.size() + need.size() / sizeof(unsigned);
+        std::vector<unsigned> lists(2 * tables, 0u);
+        std::copy(lut.begin(), lut.end(), lists.begin());
+        std::memcpy(lists.data() + lut.size(), need.data(), need.size());
+        d_lut = device_alloc<unsigned>(fixed_owned, lists.size());
+        d_need = reinterpret_cast<unsigned char*>(d_lut + lut.size());
+        d_lut_empty = d_lut + tables;
+        d_need_empty = d_need + tables * sizeof(unsigned);
         std::vector<int> coord(static_cast<std::size_t>(P));
         for (int s = 0; s < P; ++s) {
             const auto& c = coords[static_cast<std::size_t>(s)];
@@ -730,10 +721,7 @@ struct dsx_grid {
         }
         d_coord = device_alloc<int>(fixed_owned, coord.size());
         up(d_nn, nn); up(d_nbr, nbr); up(d_recv_entry, recv_entry); up(d_sender_of, sender_of);
-        up(d_shift, shift); up(d_dir, dir); up(d_lut, lut); up(d_coord, coord);
-        up(d_lut_empty, std::vector<unsigned>(lut.size(), 0u));
-        up(d_need, need);
-        up(d_need_empty, std::vector<unsigned char>(need.size(), 0));
+        up(d_shift, shift); up(d_dir, dir); up(d_lut, lists); up(d_coord, coord);
 
         // uniform cuts (dsDecompX src/topology.cpp:63-75)
         std::vector<double> c;
@@ -766,8 +754,11 @@ struct dsx_grid {
         const std::size_t report_words = report_flags + static_cast<std::size_t>(P);
         status = device_alloc<unsigned>(fixed_owned, report_words);
         cuda_check(cudaMemset(status, 0, report_words * sizeof(unsigned)), "memset");
-        cuda_check(cudaMallocHost(reinterpret_cast<void**>(&pinned_report), report_words * sizeof(unsigned)),
+        // (the image is followed by the words that steps report through)
+        cuda_check(cudaMallocHost(reinterpret_cast<void**>(&pinned_report), (report_words + 12) * sizeof(unsigned)),
                    "cudaMallocHost");
+        pinned_status = pinned_report + report_words;
+        pinned_build = pinned_status + 4;
         call_counter = device_alloc<long long>(fixed_owned, 1);
         cuda_check(cudaMemset(call_counter, 0, sizeof(long long)), "memset");
         rebalance_result = device_alloc<double>(fixed_owned, 6);
@@ -1284,7 +1275,7 @@ struct dsx_grid {
 
     // (the fence is a word of the report block that no report holds)
     dsx::Branch emigrant_branch(bool fence) const {
-        return {emigrant_stream, emigrant_fork, emigrant_join, fence ? status + 7 : nullptr};
+        return {side_stream, fork_ev, join_ev, fence ? status + 7 : nullptr};
     }
 
     void enqueue_step(dsx_step_callback cb, void* user, cudaStream_t stream, bool build_event = false) {
