@@ -4267,15 +4267,24 @@ void launch_step_move(const Grid& G, const Arrays& A, long long src_off, long lo
     }
 }
 
+// Without `overlap` the kernels of many CTAs are launched without programmatic
+// edges.  Beside a move, on a stream of the highest priority, such an edge costs
+// more than the launch it hides: the next kernel's CTAs take the slots that the
+// move's (or another stream's) would fill and wait in them.  Three grids of 1.3M
+// particles in 8x4x4, each on its stream: 197 us a step with the edges, 188
+// without (194 on one stream each, without the branch); alone, 4M 474 / 464, 1.3M
+// 251 / 250, 0.6M 170 / 176, where the chain is longer than the move.
 void launch_step_emigrants(const Grid& G, const Arrays& A, long long src_off, long long dst_off,
-                           const Scratch& S, const int* local_imm, const int* gap, cudaStream_t s) {
+                           const Scratch& S, const int* local_imm, const int* gap, cudaStream_t s,
+                           bool overlap) {
+    overlap = overlap && !joined(s);
     const int chunk_grid = S.max_chunks < sm_count() * 4 ? S.max_chunks : sm_count() * 4;
     const size_t smem = sizeof(int) * NW * G.P;
-    pdl_launch(k_emig_hist, chunk_grid > 0 ? chunk_grid : 1, NT, smem, s, G.P, S.emig_info, S.emig_dst,
-                                                                  S.emig_hist);
-    pdl_launch(k_emig_colscan, G.P, NT, 0, s, G.P, S.emig_info, S.emig_hist, local_imm, G.status);
-    pdl_launch(k_emig_place, chunk_grid > 0 ? chunk_grid : 1, NT, smem, s,
-        G, A, src_off, dst_off, S.emig_info, S.emig_src, S.emig_dst, S.emig_hist, S.imm_base, gap);
+    launch(overlap, 1, k_emig_hist, chunk_grid > 0 ? chunk_grid : 1, NT, smem, s, G.P, S.emig_info, S.emig_dst,
+           S.emig_hist);
+    launch(!joined(s), 1, k_emig_colscan, G.P, NT, 0, s, G.P, S.emig_info, S.emig_hist, local_imm, G.status);
+    launch(overlap, 1, k_emig_place, chunk_grid > 0 ? chunk_grid : 1, NT, smem, s, G, A, src_off, dst_off,
+           S.emig_info, S.emig_src, S.emig_dst, S.emig_hist, S.imm_base, gap);
     if (S.marks) S.marks->mark(s, "emig_place");
 }
 
@@ -4318,24 +4327,22 @@ void launch_step_finish(const Grid& G, const Grid& Gn, const Arrays& A, long lon
         else immigrants(k_step_immigrants<256, 3>, 256, G.P > 16 ? 4 : 8);
         return;
     }
-    launch_step_emigrants(G, A, src_off, dst_off, S, S.imm_total, nullptr, s);
-    if (halo) launch_step_immigrant_halo(Gn, A, dst_off, ghost_off, S, s);
+    launch_step_emigrants(G, A, src_off, dst_off, S, S.imm_total, nullptr, s, !forked);
+    if (halo) launch_step_immigrant_halo(Gn, A, dst_off, ghost_off, S, s, !forked);
 }
 
 void launch_step_immigrant_halo(const Grid& Gn, const Arrays& A, long long dst_off,
-                                long long ghost_off, const Scratch& S, cudaStream_t s) {
-    const Grid& G = Gn;
+                                long long ghost_off, const Scratch& S, cudaStream_t s, bool overlap) {
+    overlap = overlap && !joined(s);
     // immigrants: masks, list ranks and ghost images over their segments
-    const int imm_grid = G.max_tiles < sm_count() * 4 ? G.max_tiles : sm_count() * 4;
-    pdl_launch(k_halo_classify, imm_grid, NT, 0, s, Gn, S.imm_tiles, S.imm_tile_start + G.P,
-                                            A.d[0] + dst_off, A.d[1] + dst_off, A.d[2] + dst_off,
-                                            S.mask, S.cnt2, S.stride);
-    pdl_launch(k_scan_counters, kHaloCounters, 1024, 0, s, S.cnt2, S.pre2, S.stride,
-                                                   S.imm_tile_start + G.P);
-    pdl_launch(k_halo_scatter, imm_grid, NT, 0, s, Gn, A, dst_off, ghost_off, S.imm_tiles,
-                                           S.imm_tile_start + G.P, S.mask, S.pre2, S.stride,
-                                           S.cbase_imm, S.ghost_owner, S.ghost_entry, S.bowner,
-                                           S.boff, S.bslot, S.bfirst);
+    const int imm_grid = Gn.max_tiles < sm_count() * 4 ? Gn.max_tiles : sm_count() * 4;
+    const int* ntiles = S.imm_tile_start + Gn.P;
+    launch(overlap, 1, k_halo_classify, imm_grid, NT, 0, s, Gn, S.imm_tiles, ntiles, A.d[0] + dst_off,
+           A.d[1] + dst_off, A.d[2] + dst_off, S.mask, S.cnt2, S.stride);
+    launch(!joined(s), 1, k_scan_counters, kHaloCounters, 1024, 0, s, S.cnt2, S.pre2, S.stride, ntiles);
+    launch(overlap, 1, k_halo_scatter, imm_grid, NT, 0, s, Gn, A, dst_off, ghost_off, S.imm_tiles, ntiles,
+           S.mask, S.pre2, S.stride, S.cbase_imm, S.ghost_owner, S.ghost_entry, S.bowner, S.boff, S.bslot,
+           S.bfirst);
 }
 
 cudaError_t fork_branch(const Branch& b, cudaStream_t s) {

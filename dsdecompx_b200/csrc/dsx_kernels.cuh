@@ -160,11 +160,14 @@ bool few_tiles(const Grid& G);
 // The finish in its two parts: the emigrants' stable multi-split into the
 // next half (local_imm: emigrants expected per destination, checked; gap:
 // null, or P x P slots left before each source's group for other shards'
-// immigrants), then the immigrants' masks and ghost images.
+// immigrants), then the immigrants' masks and ghost images.  overlap: with
+// programmatic edges.
 void launch_step_emigrants(const Grid& G, const Arrays& A, long long src_off, long long dst_off,
-                           const Scratch& S, const int* local_imm, const int* gap, cudaStream_t s);
+                           const Scratch& S, const int* local_imm, const int* gap, cudaStream_t s,
+                           bool overlap = true);
 void launch_step_immigrant_halo(const Grid& Gn, const Arrays& A, long long dst_off,
-                                long long ghost_off, const Scratch& S, cudaStream_t s);
+                                long long ghost_off, const Scratch& S, cudaStream_t s,
+                                bool overlap = true);
 // A sharded step's pieces around its host-planned layout: the counter scan
 // alone, and the per-subdomain export of the scanned counters (29 P + 1 ints,
 // see k_step_export).
