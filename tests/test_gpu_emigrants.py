@@ -1,8 +1,9 @@
 """Both ways of placing emigrants (one CTA per destination up to 1,024 tiles,
 the chain of kernels beyond) and the counters around them, against the oracle:
 list lengths around the four entries a thread reads, more immigrants than one
-pass of a CTA takes, tile counts around the scan's rows, and few enough
-subdomains for copies of the immigrant counters."""
+pass of a CTA takes, and few enough
+subdomains for copies of the immigrant counters; and the scan of the tiles'
+counters around its rows."""
 import numpy as np
 import pytest
 
@@ -82,6 +83,43 @@ def test_many_emigrants_share_a_cluster(cuda, dims, n, sigma):
         assert (pair.gpu.totals()["emigrants"] > 4_096) == (n != 9_001)
     finally:
         pair.close()
+
+
+@pytest.mark.parametrize("tiles", [4_095, 4_097, 32_767, 32_770])
+def test_tile_scans_around_their_rows(cuda, tiles):
+    """A migrate of as many tiles as fill the scan's rows (4,096 tiles to a row
+    of the block, eight rows a pass), one less and a few more: every id where
+    a stable sort by destination, retained particles first, puts it."""
+    import torch
+
+    import dsdecompx_b200 as dsx
+    from test_gpu_walk_rule import Address
+
+    n, P = tiles * 512 - 700, 2    # the subdomains' last tiles are not full
+    gen = torch.Generator("cuda").manual_seed(tiles)
+    x = torch.rand(n, generator=gen, dtype=torch.float64, device="cuda")
+    source = (x >= 0.5).long()
+    order = torch.sort(source, stable=True)[1]
+    x, source = x[order], source[order]
+    counts = torch.bincount(source, minlength=P)
+    assert int(((counts + 511) // 512).sum()) in (tiles, tiles - 1)
+    ids = torch.arange(n, dtype=torch.int32, device="cuda")
+    moved = x + 0.01 * torch.randn(n, generator=gen, dtype=torch.float64, device="cuda")
+    moved = moved - torch.floor(moved)
+    half = torch.full_like(moved, 0.5)
+    grid = dsx.VirtualGrid(P, dims=(2, 1, 1), upper=(1.0, 1.0, 1.0), halo_width=0.01, particles=n,
+                           ghost_capacity=n // 8)
+    torch.cuda.synchronize()
+    arrays = {0: moved, 1: half, 2: half, 12: ids}
+    grid.upload_flat(counts.cpu().numpy(), [arrays[k].data_ptr() if k in arrays else None for k in range(13)])
+    res = grid.migrate()
+    dest = (moved >= 0.5).long()
+    want = ids[torch.sort(dest * 2 + (dest != source).long(), stable=True)[1]]
+    assert (res[:, 5] == torch.bincount(dest, minlength=P).cpu().numpy()).all()
+    v = grid.view()
+    got = torch.as_tensor(Address(grid, v.base[12] + v.owned_offset * 4, n, "i4"), device="cuda")
+    assert torch.equal(got, want)
+    grid.close()
 
 
 @pytest.mark.parametrize("program", ["emigrant_sanity", "join_sanity"])
