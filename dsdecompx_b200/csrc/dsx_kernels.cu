@@ -693,8 +693,7 @@ __device__ __forceinline__ unsigned halo_mask(const TileBounds& b, const unsigne
 
 // Adds this warp's contribution of one 32-particle group to the per-lane
 // counters (lane n < 26: send list n, lane 26: boundary owners, lane 27: images).
-__device__ __forceinline__ void count_group(unsigned m, int nn, int lane, int& acc) {
-    (void)nn;
+__device__ __forceinline__ void count_group(unsigned m, int lane, int& acc) {
     const unsigned any = __ballot_sync(0xffffffffu, m != 0);
     if (!any) return;
     // only the neighbors some lane of the warp sends to (a face particle of a
@@ -714,10 +713,11 @@ __device__ __forceinline__ void count_group(unsigned m, int nn, int lane, int& a
 // emigrant bound for subdomain `key` (-1: none) with the new owner's
 // neighbor mask `me`, counted into the owner's total, boundary, image and
 // per-list counters with one atomic per distinct destination of the warp.
-// Every lane of the warp calls it.  It pays where the emigrants of a step are
-// many and share few destinations (per-lane atomics on the same counters
-// serialise); with a few emigrants per warp the match costs more than it
-// saves, and the autotuner chooses.
+// Every lane of the warp calls it.  It pays where a tile's emigrants share few
+// destinations and the counters have few copies (8M particles in 8x8x4, fast
+// ones: 63 us of classify against 90 with an atomic per lane); with 32 copies
+// of few counters, or few emigrants a warp, the match costs more than it saves
+// (2M in 2x2x2, 25 against 21), and the autotuner chooses.
 __device__ __forceinline__ void add_immigrants(int key, unsigned me, int lane, int* total,
                                                int* bnd, int* img, int* list) {
     const unsigned peers = __match_any_sync(0xffffffffu, key);
@@ -755,7 +755,6 @@ __device__ __forceinline__ void halo_classify_tile(int g, const Grid& G,
     const int wbegin = begin + warp * 32 * ITEMS;
     const TileBounds b = halo_bounds(G, s);
     const unsigned* lut = G.lut + s * 64;
-    const int nn = G.nn[s];
     int acc = 0;
     double px[ITEMS], py[ITEMS], pz[ITEMS];
 #pragma unroll
@@ -775,7 +774,7 @@ __device__ __forceinline__ void halo_classify_tile(int g, const Grid& G,
             m = halo_mask(b, lut, px[j], py[j], pz[j]);
             mask[i] = m;
         }
-        count_group(m, nn, lane, acc);
+        count_group(m, lane, acc);
     }
     s_cnt[warp][lane] = acc;
     __syncthreads();
@@ -962,7 +961,7 @@ __device__ __forceinline__ void halo_scatter_tile(int g, const Grid& G, const Ar
     }
     int acc = 0;
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) count_group(m[j], nn, lane, acc);
+    for (int j = 0; j < ITEMS; ++j) count_group(m[j], lane, acc);
     s_cnt[warp][lane] = acc;
     if (threadIdx.x < kHaloCounters) {
         const int k = threadIdx.x;
@@ -4512,8 +4511,8 @@ void launch_forward_fields(const Grid& G, const Arrays& A, long long owned_off,
         pdl_launch(k_forward_by_list, grid, NT, 0, s, A, owned_off, ghost_off, F, G.P * kMaxNeighbors,
                    S.halo_info, S.list_flat, S.send_base, S.ghost_owner, G.status, shape);
     } else {
-        pdl_launch(k_forward_fields, resident_grid(reinterpret_cast<const void*>(k_forward_fields), G.gcap), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
-                                                            S.ghost_owner, G.status);
+        pdl_launch(k_forward_fields, resident_grid(reinterpret_cast<const void*>(k_forward_fields), G.gcap),
+                   NT, 0, s, A, owned_off, ghost_off, F, S.halo_info, S.ghost_owner, G.status);
     }
 }
 
@@ -4530,8 +4529,8 @@ void launch_reverse_sum3(const Grid& G, double* ox, double* oy, double* oz, cons
         }
     } else {
         const int grid = S.reverse_per_sm > 0 ? sm_count() * S.reverse_per_sm : owners_grid(G);
-        pdl_launch(k_reverse_sum3, grid, NT, 0, s, S.halo_info, S.bowner, S.boff, S.bslot, S.bfirst, ox, oy, oz, gx,
-                                           gy, gz, G.status, 0, -1);
+        pdl_launch(k_reverse_sum3, grid, NT, 0, s, S.halo_info, S.bowner, S.boff, S.bslot, S.bfirst,
+                   ox, oy, oz, gx, gy, gz, G.status, 0, -1);
     }
     if (S.marks) S.marks->mark(s, "reverse_sum");
 }
@@ -4539,8 +4538,9 @@ void launch_reverse_sum3(const Grid& G, double* ox, double* oy, double* oz, cons
 void launch_reverse_fields(const Grid& G, const Arrays& A, long long owned_off,
                            long long ghost_off, const FieldOps& F, const Scratch& S,
                            cudaStream_t s) {
-    pdl_launch(k_reverse_fields, dim3(resident_grid(reinterpret_cast<const void*>(k_reverse_fields), G.ncap), F.count), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
-                                                        S.bowner, S.boff, S.bslot, S.bfirst, G.status);
+    const int blocks = resident_grid(reinterpret_cast<const void*>(k_reverse_fields), G.ncap);
+    pdl_launch(k_reverse_fields, dim3(blocks, F.count), NT, 0, s, A, owned_off, ghost_off, F, S.halo_info,
+               S.bowner, S.boff, S.bslot, S.bfirst, G.status);
 }
 
 void launch_rebalance(const Grid& G, const double* work, RebalanceParams params,
