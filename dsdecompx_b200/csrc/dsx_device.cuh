@@ -66,6 +66,7 @@ struct Grid {
     double upper[3] = {1, 1, 1};
     double extent[3] = {1, 1, 1};   // upper - lower, computed once on the host
     double width = 0.0;             // halo width
+    int edges = 1;                  // whether edges and corners have send lists
     long long ncap = 0;             // owned half length
     long long particles = 0;        // owned particles in the grid
     long long gcap = 0;             // ghost capacity

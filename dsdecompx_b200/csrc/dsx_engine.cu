@@ -560,6 +560,7 @@ struct dsx_grid {
             G.extent[a] = desc.upper[a] - desc.lower[a];
             G.cut_offset[a] = cut_offset[a];
         }
+        G.edges = desc.edges_and_corners ? 1 : 0;
         G.width = halo_width;
         G.ncap = ncap;
         G.particles = total;

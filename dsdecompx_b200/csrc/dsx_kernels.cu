@@ -4431,10 +4431,52 @@ double touched_bytes(const Grid& G, int bytes) {
     return static_cast<double>(G.particles) * bytes * (1.0 - std::pow(inner_share(G), in_atom));
 }
 
+// The share of an array's 64-byte atoms (eight particles each) that a sender's
+// send lists hold, summed over the lists of a mean cell: how often the atoms are
+// read where no list finds them in the L2.
+double lists_share(const Grid& G) {
+    double sum = 0.0;
+    for (int d = 0; d < 27; ++d) {
+        const int dir[3] = {d / 9 - 1, d / 3 % 3 - 1, d % 3 - 1};
+        double layer = 1.0, exist = 1.0;
+        int split = 0;
+        for (int a = 0; a < 3; ++a) {
+            if (!dir[a]) continue;
+            ++split;
+            if (G.dims[a] == 1) exist = 0.0;
+            if (!G.periodic[a]) exist *= (G.dims[a] - 1.0) / G.dims[a];
+            layer *= G.width * G.dims[a] / G.extent[a];
+        }
+        if (!split || (split > 1 && !G.edges)) continue;
+        sum += exist * (1.0 - std::pow(layer < 1.0 ? 1.0 - layer : 0.0, 8.0));
+    }
+    return sum;
+}
+
+// Whether a full refresh of `arrays` arrays goes tile by tile: a wide record
+// whose thick and many lists (a halo of several percent of the cell, few large
+// subdomains) would read each atom twice and more, because the lists of the
+// senders in flight exceed the L2 together.  A tile's owners are read once,
+// for a latency chain per tile that only so many re-reads outweigh.  The line is
+// fitted: touched bytes x lists' share / sqrt(subdomains), in MiB, for 11 arrays of
+// 100 B, list by list / tile by tile: 2x2x2, 8M, halo 8% of the cell (943) 395 /
+// 446 us, 15% (1768) 908 / 759, 16M, 5% (1130) 709 / 670, 8% (1888) 1216 / 863; 2x2x1,
+// 16M, 5% (889) 536 / 647, 8% (1539) 771 / 705; 4x4x2, 16M, 8% (943) 659 / 860, 27M, 8% (1586) 1730 / 1441; 3x2x2,
+// 8M, 15% (1460) 734 / 762.  With lists in one dimension only (share below 2) it
+// never pays, and records of fewer arrays gain little.
+bool walk_by_tile(const Grid& G, int arrays, double touched) {
+    const double share = lists_share(G);
+    return arrays >= 9 && share >= 2.0 && touched * share > std::sqrt(static_cast<double>(G.P)) * (1100ll << 20);
+}
+
 void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, long long ghost_off,
                          bool positions_only, const Scratch& S, cudaStream_t s, int ctas_per_sm) {
     const int stage = refresh_stage_bytes(A, positions_only);
-    const bool tiles = S.refresh_kind == 2;
+    double touched = (positions_only ? 3 : 6) * touched_bytes(G, 8);
+    if (!positions_only)
+        for (int f = 0; f < A.f.count; ++f) touched += touched_bytes(G, A.f.bytes[f]);
+    const bool tiles = S.refresh_kind == 2 || (S.refresh_kind == 3 && !positions_only &&
+                                                walk_by_tile(G, 6 + A.f.count, touched));
     if (tiles && stage <= kStagedMaxBytes) {
         static bool attribute_set = false;   // once per process (one device per process)
         static std::mutex lock;
@@ -4475,9 +4517,6 @@ void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, lo
                                                   S.bfirst, S.ghost_entry);
         return;
     }
-    double touched = (positions_only ? 3 : 6) * touched_bytes(G, 8);
-    if (!positions_only)
-        for (int f = 0; f < A.f.count; ++f) touched += touched_bytes(G, A.f.bytes[f]);
     const bool by_list = S.refresh_kind == 3 && walk_by_list(G, touched, kRefreshShare);
     // in slot order: positions, and records of few fields
     if (!by_list && (positions_only || A.f.count < kRowFields)) {

@@ -213,3 +213,17 @@ def test_reverse_sum_of_more_owners_than_expected(cuda):
         assert not torch.equal(results[0][a], torch.full_like(owned[a], 0.5))
         assert torch.equal(results[0][a], results[1][a]), a
     grid.close()
+
+
+@pytest.mark.parametrize("dims,n,halo,periodic,by_tile", [
+    ((2, 2, 2), 6_500_003, 0.2, (True, True, True), True),      # thick lists of few large subdomains
+    ((3, 2, 2), 9_000_001, 0.18, (True, False, True), True),
+    ((2, 1, 1), 12_000_017, 0.2, (True, True, True), False),    # lists in one dimension
+    ((2, 2, 2), 6_500_003, 0.05, (True, True, True), False),    # thin ones
+], ids=["thick", "open", "one_axis", "thin"])
+def test_thick_lists_of_wide_records_go_tile_by_tile(cuda, dims, n, halo, periodic, by_tile):
+    grid, ghosts = make(dims, n, halo, periodic, FLUID)
+    names = kernels(lambda: grid.exchange_halo(results=False))
+    assert any("k_halo_refresh_staged" in k for k in names) == by_tile, names
+    check_walks(grid, ghosts, FLUID, False)
+    grid.close()
