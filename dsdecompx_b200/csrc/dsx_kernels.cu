@@ -4395,42 +4395,6 @@ int refresh_stage_bytes(const Arrays& A, bool positions_only) {
     return bytes;
 }
 
-// Whether a walk whose arrays hold boundary particles in `touched` bytes of
-// DRAM atoms goes list by list.
-//
-// Slot order reads a sender's 64-byte atoms again for each of its receivers.
-// Those follow one another along the faster axes; the two along the slowest
-// split axis lie a whole plane of subdomains away, and between them the walk
-// touches about one plane's share of what it reads in all.  While that share,
-// or all of it, stays in the L2 (126 MB), slot order reads every atom once too,
-// and the list walk only adds its searches; so a walk goes list by list where
-// the touched bytes exceed the L2 and a plane's share exceeds a quarter of it
-// (`share`: the forward exchange in slot order holds four times the warps, and
-// its line is higher).
-//
-// Measured, slot order / list by list in us (touched MB, a plane's share).
-// Positions: 3M in 4x4x4 (72, 18) 35.5 / 39.7; 6M in 2x2x2 (141, 70) 114 / 70, in
-// 4x4x4 (141, 35) 99 / 70; 16M in 8x8x4, thin halo (148, 18) 55 / 59, 8% halo
-// (384, 48) 284 / 174.  Full refresh of 104 B: 1.5M in 2x2x2, thin (60, 30) 16.9 /
-// 19.1, 8% halo (153, 76) 78 / 62; 16M in 8x8x4, thin (640, 80) 211 / 186.
-// Forward: 16M of 8 B in 8x8x4 (128, 16) 49 / 71; 6M of 32 B in 8x8x4 (188, 24)
-// 51 / 59, in 4x4x4 (188, 47) 71 / 58; 6M of 56 B in 2x2x2 (336, 168) 226 / 129.
-bool walk_by_list(const Grid& G, double touched, long long share) {
-    int planes = 1;
-    for (int a = 0; a < 3 && planes == 1; ++a) planes = G.dims[a];
-    return touched > (128ll << 20) && touched > static_cast<double>(share) * planes;
-}
-// fields from which a refresh in slot order goes row by row (k_halo_refresh_slots)
-constexpr int kRowFields = 3;
-constexpr long long kRefreshShare = 32ll << 20, kForwardShare = 40ll << 20;
-
-// The bytes of 64-byte atoms that hold a boundary particle, of an array of
-// `bytes` a particle.
-double touched_bytes(const Grid& G, int bytes) {
-    const double in_atom = bytes < 64 ? 64.0 / bytes : 1.0;
-    return static_cast<double>(G.particles) * bytes * (1.0 - std::pow(inner_share(G), in_atom));
-}
-
 // The share of an array's 64-byte atoms (eight particles each) that a sender's
 // send lists hold, summed over the lists of a mean cell: how often the atoms are
 // read where no list finds them in the L2.
@@ -4453,20 +4417,65 @@ double lists_share(const Grid& G) {
     return sum;
 }
 
+// Whether a walk whose arrays hold boundary particles in `touched` bytes of
+// DRAM atoms goes list by list.
+//
+// Slot order reads a sender's 64-byte atoms again for each of its receivers.
+// Those follow one another along the faster axes; the two along the slowest
+// split axis lie a whole plane of subdomains away, and between them the walk
+// touches about one plane's share of what it reads in all.  While that share,
+// or all of it, stays in the L2 (126 MB), slot order reads every atom once too,
+// and the list walk only adds its searches; so a walk goes list by list where
+// the touched bytes exceed the L2 and a plane's share exceeds a quarter of it
+// (`share`: the forward exchange in slot order holds four times the warps, and
+// its line is higher).  Along one split axis a sender has two lists, and slot
+// order is list order: there is something to find in the L2 only where the two
+// overlap (8M of 48 B in 2x1x1, halo 8% of the cell, lists' share 0.97: 89 / 99 us,
+// 15%, 1.46: 140 / 133).
+//
+// Measured, slot order / list by list in us (touched MB, a plane's share).
+// Positions: 3M in 4x4x4 (72, 18) 35.5 / 39.7; 6M in 2x2x2 (141, 70) 114 / 70, in
+// 4x4x4 (141, 35) 99 / 70; 16M in 8x8x4, thin halo (148, 18) 55 / 59, 8% halo
+// (384, 48) 284 / 174.  Full refresh of 104 B: 1.5M in 2x2x2, thin (60, 30) 16.9 /
+// 19.1, 8% halo (153, 76) 78 / 62; 16M in 8x8x4, thin (640, 80) 211 / 186.
+// Forward: 16M of 8 B in 8x8x4 (128, 16) 49 / 71; 6M of 32 B in 8x8x4 (188, 24)
+// 51 / 59, in 4x4x4 (188, 47) 71 / 58; 6M of 56 B in 2x2x2 (336, 168) 226 / 129.
+bool walk_by_list(const Grid& G, double touched, long long share) {
+    int planes = 1, split = 0;
+    for (int a = 0; a < 3; ++a) {
+        if (planes == 1) planes = G.dims[a];
+        split += G.dims[a] > 1;
+    }
+    if (split == 1 && lists_share(G) < 1.2) return false;
+    return touched > (128ll << 20) && touched > static_cast<double>(share) * planes;
+}
+// fields from which a refresh in slot order goes row by row (k_halo_refresh_slots)
+constexpr int kRowFields = 3;
+constexpr long long kRefreshShare = 32ll << 20, kForwardShare = 40ll << 20;
+
+// The bytes of 64-byte atoms that hold a boundary particle, of an array of
+// `bytes` a particle.
+double touched_bytes(const Grid& G, int bytes) {
+    const double in_atom = bytes < 64 ? 64.0 / bytes : 1.0;
+    return static_cast<double>(G.particles) * bytes * (1.0 - std::pow(inner_share(G), in_atom));
+}
+
 // Whether a full refresh of `arrays` arrays goes tile by tile: a wide record
 // whose thick and many lists (a halo of several percent of the cell, few large
-// subdomains) would read each atom twice and more, because the lists of the
-// senders in flight exceed the L2 together.  A tile's owners are read once,
-// for a latency chain per tile that only so many re-reads outweigh.  The line is
-// fitted: touched bytes x lists' share / sqrt(subdomains), in MiB, for 11 arrays of
-// 100 B, list by list / tile by tile: 2x2x2, 8M, halo 8% of the cell (943) 395 /
-// 446 us, 15% (1768) 908 / 759, 16M, 5% (1130) 709 / 670, 8% (1888) 1216 / 863; 2x2x1,
-// 16M, 5% (889) 536 / 647, 8% (1539) 771 / 705; 4x4x2, 16M, 8% (943) 659 / 860, 27M, 8% (1586) 1730 / 1441; 3x2x2,
-// 8M, 15% (1460) 734 / 762.  With lists in one dimension only (share below 2) it
-// never pays, and records of fewer arrays gain little.
+// subdomains) would read each atom twice and more, because what one sender's
+// lists read does not stay in the L2 from the first to the last.  A tile's owners
+// are read once, for a latency chain per tile that only so many re-reads outweigh.
+// The line is fitted: touched MiB x (lists' share / subdomains)^0.7; with 11 arrays
+// of 100 B, list by list / tile by tile in us: 2x2x2, halo 8% of the cell, 8M (426)
+// 395 / 446, 16M (851) 1216 / 863, 5%, 16M (583) 709 / 670, 15%, 5M (416) 388 / 488, 8M
+// (663) 908 / 759, 25%, 3M (362) 372 / 424; 3x2x2, 5%, 16M (438) 595 / 672, 15%, 8M (504)
+// 734 / 762, 8%, 16M (639) 1113 / 862; 4x4x2, 5%, 27M (372) 1000 / 1101, 8%, 27M (543)
+// 1730 / 1441; 2x2x1, 8%, 8M (463) 355 / 361, 16M (927) 771 / 705.  With lists in one
+// dimension only (share below 2) it never pays, and records of fewer arrays gain
+// little.
 bool walk_by_tile(const Grid& G, int arrays, double touched) {
     const double share = lists_share(G);
-    return arrays >= 9 && share >= 2.0 && touched * share > std::sqrt(static_cast<double>(G.P)) * (1100ll << 20);
+    return arrays >= 9 && share >= 2.0 && touched * std::pow(share / G.P, 0.7) > (490ll << 20);
 }
 
 void launch_halo_refresh(const Grid& G, const Arrays& A, long long owned_off, long long ghost_off,

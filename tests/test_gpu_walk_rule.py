@@ -141,9 +141,10 @@ def test_list_walk_splits_by_the_plan(cuda, n, halo, ghost_capacity, fields, pos
     # what slot order touches between two of a sender's receivers fits the L2
     ((8, 8, 4), 4_000_000, 0.05, [], "positions"),
     ((2, 2, 2), 4_000_000, 0.01, [], "positions"),
+    ((2, 1, 1), 12_000_000, 0.08, [], "positions"),
     ((8, 8, 4), 6_000_000, 0.08, [("c", "uint32", 2), ("d", "uint64", 2), ("f", "float64", 1)], "forward"),
     ((2, 2, 2), 6_000_000, 0.01, [("c", "uint32", 2), ("d", "uint64", 2), ("f", "float64", 1)], "forward"),
-], ids=["plane", "thin", "forward_plane", "forward_thin"])
+], ids=["plane", "thin", "one_axis", "forward_plane", "forward_thin"])
 def test_small_reuse_distances_keep_slot_order(cuda, dims, n, halo, fields, call):
     grid, _ = make(dims, n, halo, (True, True, True), fields)
     if call == "positions":
