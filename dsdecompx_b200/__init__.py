@@ -564,8 +564,8 @@ class VirtualGrid:
         """Refresh walk: "ghosts" (each ghost's owner gathered, in slot order),
         "owners" (each boundary owner once), "tiles" (each tile's owners
         staged whole) or "auto" (the default: as ghosts, list by list where
-        the copied arrays exceed the L2); True / False stand for "owners" /
-        "ghosts"."""
+        the owners' repeated reads would leave the L2, as tiles where the
+        lists' would too); True / False stand for "owners" / "ghosts"."""
         if isinstance(kind, bool):
             kind = "owners" if kind else "ghosts"
         _check(self.L.dsx_grid_set_refresh_kind(self.h, self.REFRESH_KINDS[kind]))

@@ -3974,9 +3974,9 @@ double inner_share(const Grid& G) {
 // GPU works in one narrow window of the plan that moves along, and what the
 // window's gathers share stays in the L2; the passes of one resident wave
 // spread over the plan as fast and slow CTAs drift apart.  16M clustered
-// particles, one wave / 32 / 64 / 128 CTAs per SM: reverse sum 155 / 138 / 134 /
-// 135 us (8M 73 / 63 / 63 / 71), positions by list 136 / 113 / 114 / 114, seven
-// arrays 265 / 222 / 221 / 223.
+// particles, eight (the walks: one wave) / 32 / 64 / 128 CTAs per SM: reverse sum
+// 155 / 138 / 134 / 135 us (8M 73 / 63 / 63 / 71), positions by list 136 / 113 / 114 /
+// 114, seven arrays 265 / 222 / 221 / 223.
 constexpr int kWindowPerSm = 32;
 
 int window_grid(long long items) {

@@ -85,9 +85,10 @@ struct Scratch {
                                   // 3: staged without forces, 0: direct reads
     int refresh_kind = 3;         // refresh walk: 0 ghost by ghost in slot order, 1 owner by owner
                                   // (the CSR), 2 tile by tile with the owners staged (when the
-                                  // stage fits), 3 ghost by ghost, sender by sender and list by
-                                  // list where the copied arrays exceed the L2, else as 0
-    int reverse_per_sm = 0;       // CTAs per SM of the reverse sum; 0: up to 32, one owner per thread
+                                  // stage fits), 3 ghost by ghost: as 0, or sender by sender and
+                                  // list by list (walk_by_list), or as 2 (walk_by_tile)
+    int reverse_per_sm = 0;       // CTAs per SM of the reverse sum; 0: up to 32, one expected owner
+                                  // per thread
 };
 
 void launch_layout(const Grid& G, const int* n, int* obase, int* tile_start, int4* tiles,

@@ -271,11 +271,12 @@ int dsx_grid_end_halo_exchange(dsx_grid* grid, void* stream, long long* results)
  * writing all its images; 2 tile by tile, the tile's owners brought into
  * shared memory whole and the images written in ghost-slot order (a record
  * whose copied arrays exceed 100 KB per tile falls back to 0); 3 (the
- * default) ghost by ghost, in slot order while the owned arrays that it
- * copies fit the L2 cache, else sender by sender and list by list, so that
- * every list finds its sender's particles in the cache.  All write the same
- * values; DSX_E_INVALID
- * for another kind. */
+ * default) ghost by ghost: in slot order while what it reads between two of
+ * a sender's receivers stays in the L2 cache, else sender by sender and list
+ * by list, so that every list finds its sender's particles in the cache; and
+ * tile by tile for a full refresh of nine arrays or more whose lists are too
+ * many and too thick for that.  All write the same values; DSX_E_INVALID for
+ * another kind. */
 int dsx_grid_set_refresh_kind(dsx_grid* grid, int kind);
 
 /* CTAs per SM that begin_halo_exchange's refresh may occupy (0, the default:
